@@ -54,15 +54,16 @@ def _state(solver):
 # -- metrics ------------------------------------------------------------------------
 def _run_metrics(solver, threshold: float):
     torch = _torch()
-    res = torch.zeros(ctypes.sizeof(_lib.Metrics), dtype=torch.uint8, device=solver.device)
-    gs = torch.zeros(solver.N, dtype=torch.float64, device=solver.device)
+    # the reductions and the grain sums share one buffer, read back in one copy
+    size = ctypes.sizeof(_lib.Metrics)
+    res = torch.empty(size + 8 * solver.N, dtype=torch.uint8, device=solver.device)
     front = torch.empty(solver.nx * solver.ny, dtype=torch.float32, device=solver.device)
     rc = _lib.lib().mpf3d_compact_metrics(*_state(solver), solver.slots, solver.N, solver.nx, solver.ny, solver.nz,
-                                          float(threshold), res.data_ptr(), gs.data_ptr(), front.data_ptr(),
+                                          float(threshold), res.data_ptr(), res.data_ptr() + size, front.data_ptr(),
                                           solver._stream())
     _lib.check(rc, "compact_metrics")
-    m = _lib.Metrics.from_buffer_copy(res.cpu().numpy().tobytes())
-    return m, gs.cpu().numpy(), front
+    host = res.cpu().numpy()
+    return _lib.Metrics.from_buffer_copy(host[:size].tobytes()), host[size:].view(np.float64), front
 
 
 def metrics(solver, threshold: float = 0.5, runtime_s: float = 0.0) -> dict:
