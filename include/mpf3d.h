@@ -487,6 +487,24 @@ int mpf3d_gemm_bf16_mma(int M, int N, int K, const uint16_t *A, int64_t sam, int
                         int64_t sbk, int64_t sbn, const float *bias, int act, float *Z, void *Y, int ldy,
                         int y_bf16, int beta, void *stream);
 
+/* The surrogate network 16 -> 256 -> 256 -> 256 -> 2 (SiLU between layers) on
+ * M rows in one launch: x BF16 [M][16], w16 and w its parameters W0 b0 W1 b1
+ * W2 b2 W3 b3 (W [out][in]) in BF16 (the matrices) and FP32 (the biases), out
+ * FP32 [M][2].  Z (FP32 [3][64][M][4]: layer, four columns, row) and Y (BF16
+ * [3][M][256]), or both NULL, receive the pre-activations and activations
+ * that the backward pass needs.  Arrays 16-byte aligned (out 8).  err as
+ * mpf3d_gemm_bf16. */
+int mpf3d_mlp_forward(int M, const uint16_t *x, const uint16_t *w16, const float *w, float *Z, uint16_t *Y,
+                      float *out, int32_t *err, void *stream);
+
+/* Gradients of all its parameters into g (the layout of w), given the gradient
+ * dout FP32 [M][2] of the outputs and what the forward pass kept.  Columns
+ * live_inputs.. of dW0 (padding of the input) become 0.  Scratch: dz BF16
+ * [3*256 + 8] * M, partial FP32 [4 * ceil(M / 128)][3][256]. */
+int mpf3d_mlp_backward(int M, const uint16_t *x, const uint16_t *w16, const float *Z, const uint16_t *Y,
+                       const float *dout, uint16_t *dz, float *partial, float *g, int live_inputs, int32_t *err,
+                       void *stream);
+
 /* dZ = dY * act'(Z) elementwise; outputs BF16 and/or FP32 (each nullable). */
 int mpf3d_act_backward(const float *dY, const float *Z, int act, int64_t n, uint16_t *dZ16, float *dZ32,
                        void *stream);

@@ -33,6 +33,7 @@ SOURCES = [
     ("compact.cu", ["-prec-sqrt=false"]),
     ("observe.cu", []),
     ("mlp.cu", []),
+    ("mlp_net.cu", []),
 ]
 
 

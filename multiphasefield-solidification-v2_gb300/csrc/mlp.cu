@@ -14,37 +14,18 @@
 // accumulator in tensor memory); transposed operands (the gradients) use
 // mma.sync.m16n8k16 (BF16 in, FP32 accumulate) from shared memory tiles:
 // 64 x 64 output tile per CTA, 4 warps of 32 x 32, k step 32.
-#include <cuda.h>
-#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
 
-#include <mutex>
-
 #include "mpf3d.h"
 #include "mpf3d_internal.h"
+#include "tcgen05.cuh"
 
 namespace mpf3d {
 namespace mlp {
 
 constexpr int BM = 64, BN = 64, BK = 32, PAD = 8;
-
-__device__ __forceinline__ float bf16_to_f32(uint16_t h) { return __uint_as_float((uint32_t)h << 16); }
-
-// round to nearest even (finite inputs)
-__device__ __forceinline__ uint16_t f32_to_bf16(float f) {
-    uint32_t u = __float_as_uint(f);
-    if ((u & 0x7f800000u) == 0x7f800000u) return (uint16_t)(u >> 16);  // inf / nan
-    u += 0x7fffu + ((u >> 16) & 1u);
-    return (uint16_t)(u >> 16);
-}
-
-__device__ __forceinline__ float silu(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
-__device__ __forceinline__ float silu_grad(float z) {
-    const float s = 1.0f / (1.0f + __expf(-z));
-    return s * (1.0f + z * (1.0f - s));
-}
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
     asm volatile(
@@ -239,56 +220,6 @@ namespace tc5 {
 constexpr int TM = 128;
 constexpr int MAX_N = 256;
 constexpr int MAX_K = 256;
-// bound of every mbarrier wait (nanoseconds of %globaltimer); a wait that
-// runs out aborts the CTA's work and reports MPF3D_DEV_GEMM_ABORT
-constexpr uint64_t WAIT_LIMIT_NS = 1000000000ull;
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// shared-memory matrix descriptor: start address, leading and stride byte
-// offsets (all >> 4), descriptor version 1, no swizzle
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | ((uint64_t)1 << 46);
-}
-
-// instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B,
-// both K-major, N >> 3 and M >> 4
-__host__ __device__ __forceinline__ uint32_t instr_desc(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
-__device__ __forceinline__ uint64_t global_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// waits for the phase `parity` of an mbarrier to complete, for at most
-// limit_ns; false if it did not
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint64_t limit_ns = WAIT_LIMIT_NS) {
-    const uint64_t t0 = global_ns();
-    while (true) {
-        uint32_t ok;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.b32 %0, 1, 0, p;\n}\n"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (ok) return true;
-        if (global_ns() - t0 > limit_ns) return false;
-    }
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-}
-
 // Stages rows x K of an operand into the K-major core-matrix layout:
 // element (r, k) is src[r * s_row + k * s_k]; rows at or past rows_valid
 // and columns at or past K_valid are zero.  With s_k == 1 (K contiguous in
@@ -510,42 +441,6 @@ namespace tma {
 constexpr int STAGES = 4;
 constexpr int ATOM_K = 64;                    // bf16 elements per 128-byte swizzled row
 constexpr int A_STAGE_BYTES = TM * ATOM_K * 2;  // 16 KB
-
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t addr) {
-    // K-major, 128-byte swizzle: 8-row groups 1024 bytes apart (stride byte
-    // offset); the leading byte offset is unused by this layout
-    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
-           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-}
-
-__device__ __forceinline__ void arrive_expect(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tma_load(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n" ::"r"(
-            dst),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-}
-
-__device__ __forceinline__ void umma(uint32_t tmem, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t accum) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-        "l"(ad), "l"(bd), "r"(idesc), "r"(accum)
-        : "memory");
-}
-
-__device__ __forceinline__ void commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar)
-                 : "memory");
-}
 
 __global__ void __launch_bounds__(320, 1) gemm_kernel(const __grid_constant__ CUtensorMap map_x,
                                                       const __grid_constant__ CUtensorMap map_w, int M, int N, int K,
@@ -798,36 +693,6 @@ static bool tc5_shape_ok(int M, int N, int K, const uint16_t *A, int64_t lda, co
     return M > 0 && N > 0 && N <= mpf3d::mlp::tc5::MAX_N && K >= 16 && K <= mpf3d::mlp::tc5::MAX_K && K % 16 == 0 &&
            lda >= K && ldb >= K && lda % 8 == 0 && ldb % 8 == 0 && ((uintptr_t)A & 15u) == 0 &&
            ((uintptr_t)B & 15u) == 0;
-}
-
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link
-// dependency on libcuda)
-static PFN_cuTensorMapEncodeTiled_v12000 encode_tiled() {
-    static std::once_flag once;
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    std::call_once(once, [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-                cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    });
-    return fn;
-}
-
-// 2-D map of a row-major BF16 matrix [rows][K] (row pitch ld elements):
-// boxes of 64 x box_rows, 128-byte swizzle, rows past the end read as zero
-static bool make_map(CUtensorMap *map, const uint16_t *base, int rows, int K, int64_t ld, int box_rows) {
-    PFN_cuTensorMapEncodeTiled_v12000 fn = encode_tiled();
-    if (!fn) return false;
-    cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1u, 1u};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<uint16_t *>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 // the pipelined kernel (K a multiple of 64); hold_producer != 0 only in the

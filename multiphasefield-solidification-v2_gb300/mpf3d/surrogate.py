@@ -4,12 +4,11 @@ orientations, the undercooling and the anisotropy strength to the growth
 velocity ratio and the grain-boundary inclination.
 
 Weights are stored in FP32 (Adam master copy) and BF16 (the copy the
-tensor-core GEMMs read); every matrix product runs in libmpf3d's
-`mpf3d_gemm_bf16` on the fifth-generation tensor cores (tcgen05, FP32
-accumulate in tensor memory): the forward products X W^T on the TMA-fed
-pipelined kernel, the gradients dZ W and dZ^T X on the kernel that gathers
-transposed operands into shared memory.  The activation derivative, loss and
-Adam run in its elementwise kernels.  Torch provides device memory only.
+tensor cores read).  The forward pass is one kernel that takes 128 rows through
+all layers (`mpf3d_mlp_forward`), the backward pass two: the chain of input
+gradients and all weight gradients (`mpf3d_mlp_backward`), on the
+fifth-generation tensor cores (tcgen05, FP32 accumulate in tensor memory).
+Loss and Adam are elementwise kernels.  Torch provides device memory only.
 
 No reference counterpart: the reference has no learned component; it scans
 orientations one simulation at a time (run_orientation_scan_3d.py:686-841).
@@ -160,19 +159,6 @@ class Surrogate:
     def _bf16(self, x, y):
         _lib.check(_lib.lib().mpf3d_f32_to_bf16(x.data_ptr(), y.data_ptr(), x.numel(), self._s()), "f32_to_bf16")
 
-    def _W(self, layer, bf16=True):
-        o, ob = self.offsets[layer]
-        K, N, _ = LAYERS[layer]
-        buf = self.w16 if bf16 else self.w
-        return buf.narrow(0, o, N * K), self.w.narrow(0, ob, N)
-
-    def _gemm(self, M, N, K, A, sam, sak, B, sbk, sbn, bias, act, Z, Y, ldy, y_bf16, beta=0):
-        rc = _lib.lib().mpf3d_gemm_bf16(M, N, K, A.data_ptr(), sam, sak, B.data_ptr(), sbk, sbn,
-                                        bias.data_ptr() if bias is not None else None, act,
-                                        Z.data_ptr() if Z is not None else None, Y.data_ptr(), ldy, int(y_bf16),
-                                        beta, self.gemm_err.data_ptr(), self._s())
-        _lib.check(rc, "gemm_bf16")
-
     def prepare(self, X: np.ndarray):
         """[M, <=16] float features -> zero-padded BF16 device input [M, 16]."""
         t = self.torch
@@ -190,51 +176,29 @@ class Surrogate:
         backward pass needs."""
         t = self.torch
         M = x16.shape[0]
-        h = x16
-        saved = [x16]
-        for layer, (K, N, act) in enumerate(LAYERS):
-            W16, b = self._W(layer)
-            last = layer == len(LAYERS) - 1
-            Z = t.empty((M, N), dtype=t.float32, device=self.device) if (keep and act) else None
-            Y = t.empty((M, N), dtype=t.float32 if last else t.int16, device=self.device)
-            self._gemm(M, N, K, h, K, 1, W16, 1, K, b, act, Z, Y, N, not last)
-            saved.append((Z, Y))
-            h = Y
+        out = t.empty((M, OUT), dtype=t.float32, device=self.device)
+        Z = t.empty((3, HIDDEN // 4, M, 4), dtype=t.float32, device=self.device) if keep else None
+        Y = t.empty((3, M, HIDDEN), dtype=t.int16, device=self.device) if keep else None
+        rc = _lib.lib().mpf3d_mlp_forward(M, x16.data_ptr(), self.w16.data_ptr(), self.w.data_ptr(),
+                                          Z.data_ptr() if keep else None, Y.data_ptr() if keep else None,
+                                          out.data_ptr(), self.gemm_err.data_ptr(), self._s())
+        _lib.check(rc, "mlp_forward")
         if keep:
-            self._saved = saved
-        return h
+            self._saved = (x16, Z, Y)
+        return out
 
     def backward(self, dout) -> None:
         """Gradients of the loss w.r.t. all parameters into self.g, given the
         FP32 gradient w.r.t. the outputs [M, 2]."""
         t = self.torch
-        L = _lib.lib()
-        saved = self._saved
+        x16, Z, Y = self._saved
         M = dout.shape[0]
-        dY = dout
-        for layer in range(len(LAYERS) - 1, -1, -1):
-            K, N, act = LAYERS[layer]
-            Z, _ = saved[layer + 1]
-            Hin = saved[layer] if layer == 0 else saved[layer][1]
-            dZ16 = t.empty((M, N), dtype=t.int16, device=self.device)
-            dZ32 = t.empty((M, N), dtype=t.float32, device=self.device)
-            _lib.check(L.mpf3d_act_backward(dY.data_ptr(), Z.data_ptr() if Z is not None else None, act, M * N,
-                                            dZ16.data_ptr(), dZ32.data_ptr(), self._s()), "act_backward")
-            o, ob = self.offsets[layer]
-            gW = self.g.narrow(0, o, N * K)
-            gb = self.g.narrow(0, ob, N)
-            # dW[n][k] = sum_m dZ[m][n] Hin[m][k]
-            self._gemm(N, K, M, dZ16, 1, N, Hin, K, 1, None, 0, None, gW, K, False)
-            _lib.check(L.mpf3d_colsum(dZ32.data_ptr(), M, N, N, gb.data_ptr(), self._s()), "colsum")
-            if layer > 0:
-                W16, _ = self._W(layer)
-                dH = t.empty((M, K), dtype=t.float32, device=self.device)
-                # dH[m][k] = sum_n dZ[m][n] W[n][k]
-                self._gemm(M, K, N, dZ16, N, 1, W16, K, 1, None, 0, None, dH, K, False)
-                dY = dH
-        # the padded input columns carry no parameters
-        o, _ = self.offsets[0]
-        self.g.narrow(0, o, HIDDEN * K1).view(HIDDEN, K1)[:, IN_FEATURES + DERIVED:] = 0.0
+        dz = t.empty(M * (3 * HIDDEN + 8), dtype=t.int16, device=self.device)
+        partial = t.empty(-(-M // 128) * 4 * 3 * HIDDEN, dtype=t.float32, device=self.device)
+        rc = _lib.lib().mpf3d_mlp_backward(M, x16.data_ptr(), self.w16.data_ptr(), Z.data_ptr(), Y.data_ptr(),
+                                           dout.data_ptr(), dz.data_ptr(), partial.data_ptr(), self.g.data_ptr(),
+                                           IN_FEATURES + DERIVED, self.gemm_err.data_ptr(), self._s())
+        _lib.check(rc, "mlp_backward")
 
     def loss_and_grad(self, x16, target):
         """Weighted MSE on standardised targets; fills self.g, returns the loss."""
