@@ -152,7 +152,7 @@ int mpf3d_compact_init_owner(const int32_t *owner, int slab, const float *prof, 
 int mpf3d_compact_active_count(const uint32_t *head, const uint16_t *idx, int slots, int nx, int ny, int nz,
                                int32_t *nf, void *stream);
 
-/* One time step in FP32 (three kernels): APT rebuild (src/gpu_kernels_3d.py:462-486),
+/* One time step in FP32 (a sweep and the work-list kernels): APT rebuild (src/gpu_kernels_3d.py:462-486),
  * phase update of kernel_update_phasefield_active_3d_switchable (:683-830)
  * and the cooling of kernel_update_temp_3d (:833-838) folded into
  * T = T0z[k] - (Tm_plus_cool - T_melt).  (slots, amax) is (4, 8), (8, 16) or
@@ -162,17 +162,17 @@ int mpf3d_compact_active_count(const uint32_t *head, const uint16_t *idx, int sl
  * symmetric_normals != 0 asserts that every grain's n111 rows 4..7 are the
  * exact negatives of rows 3..0 (true for the rotated (+-1,+-1,+-1)/sqrt(3)
  * set of src/orientation_utils.py:182-212), which halves the facet search
- * (the interface kernel is built once for 4 and once for 8 normals).
+ * (the interface kernels are built once for 4 and once for 8 normals).
  * Scratch: work_items uint32[cells] (cells handed from the sweep kernel to
- * the general and interface kernels of the step) and work_count uint32[4],
+ * the work-list kernels of the step) and work_count uint32[4],
  * zeroed once before the first step; `parity` alternates 0/1 on consecutive
  * steps so no reset is needed in between.  Cells must number fewer than 2^31.
- * Streams: with anisotropy on, the interface kernel runs on a library-owned
- * second stream, beside the general kernel, forked from and joined back to
- * `stream` by events; to the caller the step is ordered on `stream` like one
+ * Streams: with anisotropy on and 2^19 cells or more, the kernel of the
+ * one-solid interface cells runs on a library-owned second stream, beside the
+ * kernels of the other lists, forked from and joined back to `stream` by events; to the caller the step is ordered on `stream` like one
  * kernel.  Each caller stream of each device gets its own second stream and
  * event pair, created by its first such call made outside a stream capture;
- * a call inside a capture before that launches both kernels on `stream`.
+ * a call inside a capture before that launches them all on `stream`.
  * Steps that callers issue on independent streams therefore stay
  * independent.  The same holds for mpf3d_compact_step_tuned,
  * mpf3d_compact_step_clocked and mpf3d_compact_step_noalloc; the batched step
@@ -181,7 +181,7 @@ int mpf3d_compact_active_count(const uint32_t *head, const uint16_t *idx, int sl
  * step. */
 /* Creates the second stream of `stream` on the current device (see
  * "Streams" above) now, so that steps captured from `stream` into a CUDA
- * graph later run their general and interface kernels side by side.  Fails
+ * graph later run their work-list kernels side by side.  Fails
  * (MPF3D_ERR_CUDA) when `stream` is being captured.  Optional: the first
  * uncaptured step on `stream` does the same. */
 int mpf3d_streams_prepare(void *stream);
@@ -199,14 +199,14 @@ int mpf3d_compact_step(const uint32_t *head, const uint16_t *idx, const float *v
 typedef struct mpf3d_tuning {
     int32_t sweep_zb;              /* cells per sweep thread along z: 2, 4 or 8 */
     int32_t sweep_by;              /* sweep block = 32 x sweep_by threads: 4, 8 or 16 */
-    int32_t general_blocks_per_sm; /* general work-list kernel: blocks per SM, 1..64 */
+    int32_t general_blocks_per_sm; /* general (or isotropic) work-list kernel: blocks per SM, 1..64 */
     int32_t general_threads;       /* and threads per block: 128 or 256 */
-    int32_t iface_blocks_per_sm;   /* interface work-list kernel: blocks per SM, 1..64 */
+    int32_t iface_blocks_per_sm;   /* pair and trio work-list kernels: blocks per SM, 1..64 */
     int32_t iface_threads;         /* and threads per block: 64 or 128 */
 } mpf3d_tuning;
 
 /* mpf3d_compact_step with an explicit launch shape (NULL: the default
- * {4, 8, 8, 256, 8, 128}), as chosen by the package's autotuner, and
+ * {4, 8, 16, 128, 16, 128}), as chosen by the package's autotuner, and
  * optional quiet-tile flags.  No reference counterpart: the reference
  * launches a fixed [4, 4, 4] block (config_3d.yaml gpu.threads_per_block)
  * over every cell.
@@ -229,10 +229,10 @@ int mpf3d_compact_step_tuned(const uint32_t *head, const uint16_t *idx, const fl
                              void *stream, const mpf3d_tuning *tuning, uint8_t *tile_flags, int options);
 
 /* options of mpf3d_compact_step_tuned */
-#define MPF3D_STEP_MULTI_LIST 1 /* interface cells whose neighbourhood holds two or more solids (decided
-                                 * from the heads) get a work list of their own at
+#define MPF3D_STEP_MULTI_LIST 1 /* interface cells whose neighbourhood holds two or more solids
+                                 * get a work list of their own at
                                  * work_items[cells .. 2*cells): work_items must then hold 2*cells
-                                 * entries and work_count 6.  Same results, fewer idle lanes. */
+                                 * entries and work_count 6.  Same results, faster. */
 
 #define MPF3D_STEP_SWEEP_TMA 2 /* the sweep stages each block's heads plus a one-cell halo in shared memory
                                 * with one TMA copy (cp.async.bulk.tensor.3d) and classifies from there;

@@ -1,14 +1,15 @@
 // compact.cu -- FP32 compact-slot stepper (throughput tier).
 //
-// A time step is three kernels that together do what the reference does in
-// three dense launches (src/gpu_kernels_3d.py:462-486 APT rebuild, :530-680
-// phase update, :833-838 cooling): a sweep writes the cells whose
-// neighbourhood holds one phase and queues the rest on work lists; a general
-// kernel and an interface kernel then rebuild each queued cell's
-// active-phase list from the stored lists of the cell and its 6 face
-// neighbours, evaluate the anisotropic interface, torque and kinetic terms
-// and the pair sums, clip, renormalise and write only the phases that stay
-// positive.
+// A time step does what the reference does in three dense launches
+// (src/gpu_kernels_3d.py:462-486 APT rebuild, :530-680 phase update, :833-838
+// cooling).  A sweep writes the cells whose neighbourhood holds one phase and
+// queues the rest on work lists; the list kernels then rebuild each queued
+// cell's active-phase list from the stored lists of the cell and its 6 face
+// neighbours, evaluate the anisotropic interface, torque and kinetic terms and
+// the pair sums, clip, renormalise and write only the phases that stay positive.
+// Small domains have one list kernel (octet_kernel), large ones one per kind of
+// cell: pair_kernel, trio_kernel, general_kernel and, for what those leave,
+// rest_kernel (isotropic_kernel alone without anisotropy).
 //
 // State layout in HBM (x fastest, so a warp of 32 threads along x reads
 // 32 consecutive entries of each array and an interface -- normal to z --
@@ -83,66 +84,6 @@ struct Facet {
     float cabs, cs, nx, ny, nz, q;
 };
 
-// When the 8 normals are 4 exact antipodal pairs with one member of each
-// pair among the first four (true for the rotated (+-1,+-1,+-1)/sqrt(3) set
-// in the reference's order; checked on the host), |cos| ties exactly within
-// a pair and the first-maximum search over 8 equals the search over 4.
-template <int NT = 8>
-__device__ __forceinline__ Facet facet_n(float3 g, const float *__restrict__ u, float g2_floor) {
-    Facet f;
-    f.q = g.x * g.x + g.y * g.y + g.z * g.z;
-    f.valid = !(f.q < g2_floor);
-    f.cabs = 0.0f; f.cs = 0.0f; f.nx = 1.0f; f.ny = 0.0f; f.nz = 0.0f;
-    if (!f.valid) return f;
-    float ig = rsqrtf(f.q);
-    float gx = g.x * ig, gy = g.y * ig, gz = g.z * ig;
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-        float ux = __ldg(u + 3 * t), uy = __ldg(u + 3 * t + 1), uz = __ldg(u + 3 * t + 2);
-        float d = gx * ux + gy * uy + gz * uz;
-        float a = fabsf(d);
-        if (a > f.cabs) {
-            f.cabs = a; f.cs = d; f.nx = ux; f.ny = uy; f.nz = uz;
-        }
-    }
-    f.cabs = fminf(f.cabs, 1.0f);
-    f.cs = fminf(fmaxf(f.cs, -1.0f), 1.0f);
-    return f;
-}
-
-// facet_n over normals already held in registers (a grain's normals are
-// loaded once per cell and reused at the 7 stencil points)
-template <int NT>
-__device__ __forceinline__ Facet facet_regs(float3 g, const float (&u)[3 * NT], float g2_floor) {
-    Facet f;
-    f.q = g.x * g.x + g.y * g.y + g.z * g.z;
-    f.valid = !(f.q < g2_floor);
-    f.cabs = 0.0f; f.cs = 0.0f; f.nx = 1.0f; f.ny = 0.0f; f.nz = 0.0f;
-    if (!f.valid) return f;
-    float ig = rsqrtf(f.q);
-    float gx = g.x * ig, gy = g.y * ig, gz = g.z * ig;
-#pragma unroll
-    for (int t = 0; t < NT; ++t) {
-        const float ux = u[3 * t], uy = u[3 * t + 1], uz = u[3 * t + 2];
-        float d = gx * ux + gy * uy + gz * uz;
-        float a = fabsf(d);
-        if (a > f.cabs) {
-            f.cabs = a; f.cs = d; f.nx = ux; f.ny = uy; f.nz = uz;
-        }
-    }
-    f.cabs = fminf(f.cabs, 1.0f);
-    f.cs = fminf(fmaxf(f.cs, -1.0f), 1.0f);
-    return f;
-}
-
-// a(theta) (calc_a_from_cos :24-30)
-__device__ __forceinline__ float calc_a(const Params &P, float c) {
-    float c2 = c * c;
-    float C = sqrtf(c2 + P.pp);
-    float S = sqrtf(fmaxf(1.0f - c2, 0.0f) + P.pp);
-    return P.mu_a * (1.0f + P.delta_a * (C + P.tan_a0 * S));
-}
-
 // a * b - c * d with one rounding error at most (Kahan's difference of
 // products); the _rn intrinsics keep the compiler from contracting the
 // error-free steps into other FMAs
@@ -198,24 +139,9 @@ __device__ __forceinline__ float calc_b(const Params &P, float3 g, const Facet &
     return P.ksi + (1.0f - P.ksi) * t * tanhf(1.0f / t);
 }
 
-// d a / d(grad phi) (da_dphixyz_A12 :304-341); returns a and the 3 components
-__device__ __forceinline__ float4 da_dgrad(const Params &P, float3 g, const Facet &f) {
-    if (!f.valid) return make_float4(0.f, 0.f, 0.f, 0.f);
-    float a = calc_a(P, f.cabs);
-    float ig = rsqrtf(f.q);
-    float ig3 = ig * ig * ig;
-    float ud = g.x * f.nx + g.y * f.ny + g.z * f.nz;
-    float c = f.cs, c2 = c * c;
-    float C = sqrtf(c2 + P.pp);
-    float S = sqrtf(fmaxf(1.0f - c2, 0.0f) + P.pp);
-    float coef = P.mu_da * (c / C - P.tan_a0 * (c / S));
-    return make_float4(a, coef * (f.nx * ig - ud * g.x * ig3), coef * (f.ny * ig - ud * g.y * ig3),
-                       coef * (f.nz * ig - ud * g.z * ig3));
-}
-
-// Work lists of a step (scratch memory owned by the caller): items[cells]
-// holds x-fastest cell indices -- cells needing the general update from the
-// front, solid-liquid interface cells from the back; count[4] holds the two
+// Work lists of a step (scratch memory owned by the caller): items holds
+// x-fastest cell indices -- cells needing the general update from the front,
+// solid-liquid interface cells from items[cells - 1] down; count[4] holds the two
 // list lengths for even and odd steps (count[2*parity + 0/1]), so the sweep
 // of one step can clear the other parity's counters without a memset.
 struct Queue {
@@ -223,8 +149,7 @@ struct Queue {
     uint32_t *__restrict__ count;
     // With split set, interface cells whose active list holds two or more
     // solids go to a third list at items[cells + ...] (counters count[4 +
-    // parity]): their warps loop over the solids, and keeping them apart
-    // from the one-solid majority spares those warps the idle iterations.
+    // parity]): the second list is then pair_kernel's.
     int split;
 };
 
@@ -260,265 +185,357 @@ __device__ __forceinline__ float lap7(const Params &P, const float (&v)[7]) {
     return __fmul_rn(__fsub_rn(s, __fmul_rn(6.0f, v[0])), P.inv_dx2);
 }
 
-// Active list of one cell: the ascending union of the stored lists of the
-// cell and its 6 neighbours (the APT rule of kernel_update_nfmf_3d for
-// phi >= 0), produced by a 7-way merge of the sorted lists, which also
-// yields every active phase's value at the 7 points without any search.
-template <int AMAX>
-struct Active {
-    int n;
-    bool ovf;
-    int ids[AMAX];
-    float vc[AMAX];   // value at the cell
-    float lap[AMAX];  // 7-point Laplacian (laplacian_3d :444-459)
-    float vL[7];      // liquid at the 7 points
-    int ts;           // index of the dominant solid (max value at the cell), -1 if none
-    float3 gs;        // its gradient at the cell
-};
-
-template <int S, int AMAX>
-__device__ __forceinline__ void gather(const In &in, const Params &P, const uint32_t (&pt)[7], Active<AMAX> &A) {
-    const uint32_t cells = P.cells32;
-    int cnt[7], pos[7], head[7];
-    uint32_t hw[7];
-#pragma unroll
-    for (int p = 0; p < 7; ++p) {
-        hw[p] = __ldg(in.head + pt[p]);
-        const int c = hcount(hw[p]);
-        cnt[p] = c < S ? c : S;
-        pos[p] = 0;
-        head[p] = cnt[p] > 0 ? hid0(hw[p]) : 0x7fffffff;
-        A.vL[p] = 0.0f;
-    }
-    A.n = 0;
-    A.ovf = false;
-    A.ts = -1;
-    A.gs = make_float3(0.f, 0.f, 0.f);
-    float maxv = -1.0f;
-    while (true) {
-        int id = head[0];
-#pragma unroll
-        for (int p = 1; p < 7; ++p) id = min(id, head[p]);
-        if (id == 0x7fffffff) break;
-        float v[7];
-#pragma unroll
-        for (int p = 0; p < 7; ++p) {
-            v[p] = 0.0f;
-            if (head[p] == id) {
-                v[p] = pos[p] == 0 ? value0(in, hw[p], pt[p]) : __ldg(in.val + (uint32_t)pos[p] * cells + pt[p]);
-                ++pos[p];
-                head[p] = pos[p] < cnt[p] ? (int)__ldg(in.idx + (uint32_t)pos[p] * cells + pt[p]) : 0x7fffffff;
-            }
-        }
-        if (A.n == AMAX) {
-            A.ovf = true;
-            break;
-        }
-        A.ids[A.n] = id;
-        A.vc[A.n] = v[0];
-        A.lap[A.n] = lap7(P, v);
-        if (id == LIQ) {
-#pragma unroll
-            for (int p = 0; p < 7; ++p) A.vL[p] = v[p];
-        } else if (v[0] > maxv) {
-            maxv = v[0];
-            A.ts = A.n;
-            A.gs = make_float3((v[1] - v[2]) * P.inv_2dx, (v[3] - v[4]) * P.inv_2dx, (v[5] - v[6]) * P.inv_2dx);
-        }
-        ++A.n;
-    }
+// a b c . x y z with the roundings fixed.  The solid-liquid terms are written
+// with explicit roundings throughout, so that every kernel that inlines them,
+// and both forms of the interface update, give the same bits.
+__device__ __forceinline__ float dot3(float a, float b, float c, float x, float y, float z) {
+    return fmaf(a, x, fmaf(b, y, __fmul_rn(c, z)));
 }
 
-// Facet-derived quantities of one grain at one stencil point: the
-// anisotropy a(theta) (calc_a_from_cos :24-30), eps^2 = (eps0 a)^2 and
-// d a / d(grad phi) (da_dphixyz_A12 :304-341).  C = sqrt(c^2+p^2) and
-// S = sqrt(max(1-c^2,0)+p^2) are shared by a and da/dc.
-struct PointTerms {
-    float e2;        // eps^2 at the point
-    float a;         // a(theta)
-    float3 da;       // d a / d(phi_x, phi_y, phi_z); zero below the floor
-    float coef;      // mu_a delta_a (c/C - tan(a0) c/S)
+// The liquid gradient (or the dominant solid's) at a stencil point.
+struct Grad {
+    float3 g;
+    float q, ig;  // squared length; 1 / length, 0 below the floor
+    bool valid;
+    __device__ __forceinline__ Grad(const Params &P, float3 g_) : g(g_) {
+        q = dot3(g.x, g.y, g.z, g.x, g.y, g.z);
+        valid = !(q < P.g2_floor);
+        ig = valid ? rsqrtf(q) : 0.0f;
+    }
 };
 
-__device__ __forceinline__ PointTerms point_terms(const Params &P, float3 g, const Facet &f, bool want_da) {
+// What one grain's facet gives at a stencil point: the best normal (first
+// maximum of |cos|; below the gradient floor cosine 0), a(theta)
+// (calc_a_from_cos :24-30), eps^2 = (eps0 a)^2 and the factor of
+// d a / d(grad phi) (da_dphixyz_A12 :304-341).  With 8 normals that are 4 exact
+// antipodal pairs, one of each pair among the first four (checked on the
+// host), |cos| ties exactly within a pair and 4 normals give the same search.
+struct PointTerms {
+    float cabs, cs, nx, ny, nz, a, e2, coef;
+};
+template <int NT>
+__device__ __forceinline__ PointTerms point_terms(const Params &P, const Grad &G, const float (&un)[3 * NT]) {
     PointTerms t;
-    if (!f.valid) {
-        t.e2 = P.e2_flat;
-        t.a = 0.0f;
-        t.da = make_float3(0.f, 0.f, 0.f);
-        t.coef = 0.0f;
-        return t;
+    t.cabs = 0.0f; t.cs = 0.0f; t.nx = 1.0f; t.ny = 0.0f; t.nz = 0.0f;
+    const float x = G.g.x * G.ig, y = G.g.y * G.ig, z = G.g.z * G.ig;
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+        const float d = dot3(x, y, z, un[3 * i], un[3 * i + 1], un[3 * i + 2]);
+        const float a = fabsf(d);
+        if (a > t.cabs) {
+            t.cabs = a; t.cs = d; t.nx = un[3 * i]; t.ny = un[3 * i + 1]; t.nz = un[3 * i + 2];
+        }
     }
-    const float c = f.cs, c2 = c * c;
-    const float C = sqrtf(c2 + P.pp);
-    const float S = sqrtf(fmaxf(1.0f - c2, 0.0f) + P.pp);
-    t.a = P.mu_a * (1.0f + P.delta_a * (C + P.tan_a0 * S));
+    t.cabs = fminf(t.cabs, 1.0f);
+    t.cs = fminf(fmaxf(t.cs, -1.0f), 1.0f);
+    const float C = sqrtf(fmaf(t.cs, t.cs, P.pp)), Sn = sqrtf(fmaxf(fmaf(-t.cs, t.cs, 1.0f), 0.0f) + P.pp);
+    t.a = P.mu_a * fmaf(P.delta_a, fmaf(P.tan_a0, Sn, C), 1.0f);
     const float e = P.eps0 * t.a;
-    t.e2 = e * e;
-    t.coef = P.mu_da * (__fdividef(c, C) - P.tan_a0 * __fdividef(c, S));
-    if (want_da) {
-        const float ig = rsqrtf(f.q);
-        const float ig3 = ig * ig * ig;
-        const float ud = g.x * f.nx + g.y * f.ny + g.z * f.nz;
-        t.da = make_float3(t.coef * (f.nx * ig - ud * g.x * ig3), t.coef * (f.ny * ig - ud * g.y * ig3),
-                           t.coef * (f.nz * ig - ud * g.z * ig3));
-    } else {
-        t.da = make_float3(0.f, 0.f, 0.f);
-    }
+    t.e2 = G.valid ? e * e : P.e2_flat;
+    t.coef = P.mu_da * fmaf(-P.tan_a0, __fdividef(t.cs, Sn), __fdividef(t.cs, C));
     return t;
 }
+// d cos / d(grad phi); 0 below the floor
+__device__ __forceinline__ float3 dcos(const Grad &G, const PointTerms &t) {
+    const float ud = __fmul_rn(dot3(G.g.x, G.g.y, G.g.z, t.nx, t.ny, t.nz), __fmul_rn(__fmul_rn(G.ig, G.ig), G.ig));
+    return make_float3(fmaf(-ud, G.g.x, __fmul_rn(t.nx, G.ig)), fmaf(-ud, G.g.y, __fmul_rn(t.ny, G.ig)),
+                       fmaf(-ud, G.g.z, __fmul_rn(t.nz, G.ig)));
+}
 
-// eps^2-weighted divergence, torque and kinetic factor of one solid grain at
-// a cell from the liquid gradient at the 7 points and the liquid's second
-// derivatives at the cell (aniso_term1_solid_3d :149-204, torque_A11_3d
-// :386-441, A13_divergence_3d :344-383, calc_b_from_cos :33-55).
-template <int NT>
-__device__ __forceinline__ void interface_terms(const Params &P, const float3 (&G)[7], const float (&vL)[7],
-                                                const float (&h2)[6], const float (&u)[3 * NT], bool torque,
-                                                float &lap_sl, float &b_sl) {
-    Facet F[7];
-    bool any = false;
-#pragma unroll
-    for (int p = 0; p < 7; ++p) {
-        F[p] = facet_regs<NT>(G[p], u, P.g2_floor);
-        any = any || F[p].valid;
+// lap_sl and b_sl of one solid at a cell from its facet there and the sums
+// over the six neighbours: flux, of (eps^2 at the cell + there)(phi_L there -
+// at the cell), and div, of the neighbours' da/d(grad phi) components along
+// their own axis, + side minus - side (aniso_term1_solid_3d :149-204,
+// torque_A11_3d :386-441 with A13_divergence_3d :344-383, calc_b_from_cos
+// :33-55).  L: liquid at the 7 points; hxy, hxz, hyz: its mixed differences.
+__device__ __forceinline__ void center_terms(const Params &P, const Grad &G, const PointTerms &t, const float (&L)[7],
+                                             float hxy, float hxz, float hyz, float flux, float div, float &lap_sl,
+                                             float &b_sl) {
+    lap_sl = __fmul_rn(flux, P.inv_2dx * P.inv_dx);
+    if (!G.valid) return;
+    if (P.use_torque) {
+        const float qq = 0.25f * P.inv_dx2;
+        const float pxx = __fadd_rn(fmaf(-2.0f, L[0], L[1]), L[2]) * P.inv_dx2;
+        const float pyy = __fadd_rn(fmaf(-2.0f, L[0], L[3]), L[4]) * P.inv_dx2;
+        const float pzz = __fadd_rn(fmaf(-2.0f, L[0], L[5]), L[6]) * P.inv_dx2;
+        const float pxy = hxy * qq, pxz = hxz * qq, pyz = hyz * qq;
+        const float qx = 2.0f * dot3(G.g.x, G.g.y, G.g.z, pxx, pxy, pxz);
+        const float qy = 2.0f * dot3(G.g.x, G.g.y, G.g.z, pxy, pyy, pyz);
+        const float qz = 2.0f * dot3(G.g.x, G.g.y, G.g.z, pxz, pyz, pzz);
+        const float3 dc = dcos(G, t);
+        const float cxx = dot3(dc.x, dc.y, dc.z, pxx, pxy, pxz);
+        const float cyy = dot3(dc.x, dc.y, dc.z, pxy, pyy, pyz);
+        const float czz = dot3(dc.x, dc.y, dc.z, pxz, pyz, pzz);
+        const float dx = __fmul_rn(t.coef, dc.x), dy = __fmul_rn(t.coef, dc.y), dz = __fmul_rn(t.coef, dc.z);
+        // da/dx . da/d(grad phi) q + a div(da/d(grad phi)) q + a da/d(grad phi) . grad q
+        const float E1 = __fmul_rn(__fmul_rn(t.coef, G.q), dot3(cxx, cyy, czz, dx, dy, dz));
+        const float E2 = fmaf(__fmul_rn(t.a, G.q), __fmul_rn(div, P.half_over_dx), E1);
+        lap_sl = fmaf(P.eps0sq, fmaf(t.a, dot3(dx, dy, dz, qx, qy, qz), E2), lap_sl);
     }
-    const float Lc = vL[0];
-    const float h = P.inv_2dx * P.inv_dx;
-    if (!any) {
-        // flat liquid everywhere: eps^2 = (eps0 a(0))^2 at all 7 points, no torque
-        const float e2 = P.e2_flat;
-        lap_sl = ((2.0f * e2) * (vL[1] - Lc) - (2.0f * e2) * (Lc - vL[2])) * h +
-                 ((2.0f * e2) * (vL[3] - Lc) - (2.0f * e2) * (Lc - vL[4])) * h +
-                 ((2.0f * e2) * (vL[5] - Lc) - (2.0f * e2) * (Lc - vL[6])) * h;
+    Facet f;
+    f.valid = true;
+    f.cabs = t.cabs; f.cs = t.cs; f.nx = t.nx; f.ny = t.ny; f.nz = t.nz; f.q = G.q;
+    b_sl = calc_b(P, G.g, f);
+}
+
+// The sums over the six neighbours in the order of the octet's shuffles.
+__device__ __forceinline__ float arm_sum(const float (&f)[7]) {
+    return __fadd_rn(__fadd_rn(f[1], __fadd_rn(f[2], f[3])), __fadd_rn(__fadd_rn(f[4], f[5]), f[6]));
+}
+
+// Liquid gradients at the 7 points and mixed second differences at the cell,
+// from the liquid vL there and at the 18 further points of the 25-point stencil
+// (offsets with |dx|+|dy|+|dz| <= 2).
+struct Stencil {
+    float3 G[7];
+    float hxy, hxz, hyz;
+    __device__ __forceinline__ Stencil(const In &in, const Params &P, int l, int m, int k, const float (&vL)[7]) {
+        const int lp = wrap_p(l, P.nx), lm = wrap_m(l, P.nx), mp = wrap_p(m, P.ny), mm = wrap_m(m, P.ny);
+        const int kp = clamp_p(k, P.nz), km = clamp_m(k, P.nz);
+        const int lpp = wrap_p(lp, P.nx), lmm = wrap_m(lm, P.nx);
+        const int mpp = wrap_p(mp, P.ny), mmm = wrap_m(mm, P.ny);
+        const int kpp = clamp_p(kp, P.nz), kmm = clamp_m(km, P.nz);
+        const float Lxpyp = liquid32(in, cidx(P, lp, mp, k)), Lxpym = liquid32(in, cidx(P, lp, mm, k));
+        const float Lxmyp = liquid32(in, cidx(P, lm, mp, k)), Lxmym = liquid32(in, cidx(P, lm, mm, k));
+        const float Lxpzp = liquid32(in, cidx(P, lp, m, kp)), Lxpzm = liquid32(in, cidx(P, lp, m, km));
+        const float Lxmzp = liquid32(in, cidx(P, lm, m, kp)), Lxmzm = liquid32(in, cidx(P, lm, m, km));
+        const float Lypzp = liquid32(in, cidx(P, l, mp, kp)), Lypzm = liquid32(in, cidx(P, l, mp, km));
+        const float Lymzp = liquid32(in, cidx(P, l, mm, kp)), Lymzm = liquid32(in, cidx(P, l, mm, km));
+        const float Lx2p = liquid32(in, cidx(P, lpp, m, k)), Lx2m = liquid32(in, cidx(P, lmm, m, k));
+        const float Ly2p = liquid32(in, cidx(P, l, mpp, k)), Ly2m = liquid32(in, cidx(P, l, mmm, k));
+        const float Lz2p = liquid32(in, cidx(P, l, m, kpp)), Lz2m = liquid32(in, cidx(P, l, m, kmm));
+        const float g2 = P.inv_2dx;
+        G[0] = make_float3((vL[1] - vL[2]) * g2, (vL[3] - vL[4]) * g2, (vL[5] - vL[6]) * g2);
+        G[1] = make_float3((Lx2p - vL[0]) * g2, (Lxpyp - Lxpym) * g2, (Lxpzp - Lxpzm) * g2);
+        G[2] = make_float3((vL[0] - Lx2m) * g2, (Lxmyp - Lxmym) * g2, (Lxmzp - Lxmzm) * g2);
+        G[3] = make_float3((Lxpyp - Lxmyp) * g2, (Ly2p - vL[0]) * g2, (Lypzp - Lypzm) * g2);
+        G[4] = make_float3((Lxpym - Lxmym) * g2, (vL[0] - Ly2m) * g2, (Lymzp - Lymzm) * g2);
+        // z neighbours sit on the clamped rows: at the top/bottom row the
+        // neighbour is the cell itself
+        G[5] = (kp == k) ? G[0] : make_float3((Lxpzp - Lxmzp) * g2, (Lypzp - Lymzp) * g2, (Lz2p - vL[0]) * g2);
+        G[6] = (km == k) ? G[0] : make_float3((Lxpzm - Lxmzm) * g2, (Lypzm - Lymzm) * g2, (vL[0] - Lz2m) * g2);
+        if (kp == k) G[5].z = (vL[5] - vL[6]) * g2;
+        if (km == k) G[6].z = (vL[5] - vL[6]) * g2;
+        hxy = (Lxpyp - Lxpym) - (Lxmyp - Lxmym);
+        hxz = (Lxpzp - Lxpzm) - (Lxmzp - Lxmzm);
+        hyz = (Lypzp - Lypzm) - (Lymzp - Lymzm);
+    }
+};
+
+// lap_sl and b_sl of one solid with the liquid gradient at the 7 points in
+// one thread.
+template <int NT>
+__device__ __forceinline__ void interface_terms(const Params &P, const Stencil &st, const float (&L)[7],
+                                                const float (&un)[3 * NT], float &lap_sl, float &b_sl) {
+    const float3 (&G)[7] = st.G;
+    const Grad g0(P, G[0]);
+    bool any = g0.valid;
+#pragma unroll
+    for (int p = 1; p < 7; ++p)
+        any = any || !(dot3(G[p].x, G[p].y, G[p].z, G[p].x, G[p].y, G[p].z) < P.g2_floor);
+    float flux[7], div[7];
+    if (!any) {  // flat liquid everywhere: eps^2 = (eps0 a(0))^2 at all 7 points, no torque
+#pragma unroll
+        for (int p = 1; p < 7; ++p) flux[p] = __fmul_rn(P.e2_flat + P.e2_flat, L[p] - L[0]);
+        lap_sl = __fmul_rn(arm_sum(flux), P.inv_2dx * P.inv_dx);
         b_sl = P.b_flat;
         return;
     }
-    const bool tq = torque && F[0].valid;
-    PointTerms T[7];
-    T[0] = point_terms(P, G[0], F[0], tq);
+    const PointTerms t0 = point_terms<NT>(P, g0, un);
 #pragma unroll
-    for (int p = 1; p < 7; ++p) T[p] = point_terms(P, G[p], F[p], tq);
-    float lv = ((T[0].e2 + T[1].e2) * (vL[1] - Lc) - (T[0].e2 + T[2].e2) * (Lc - vL[2])) * h +
-               ((T[0].e2 + T[3].e2) * (vL[3] - Lc) - (T[0].e2 + T[4].e2) * (Lc - vL[4])) * h +
-               ((T[0].e2 + T[5].e2) * (vL[5] - Lc) - (T[0].e2 + T[6].e2) * (Lc - vL[6])) * h;
-    if (tq) {
-        const float3 g0 = G[0];
-        const float q = F[0].q;
-        const float pxx = h2[0], pyy = h2[1], pzz = h2[2], pxy = h2[3], pxz = h2[4], pyz = h2[5];
-        const float qx = 2.0f * (g0.x * pxx + g0.y * pxy + g0.z * pxz);
-        const float qy = 2.0f * (g0.x * pxy + g0.y * pyy + g0.z * pyz);
-        const float qz = 2.0f * (g0.x * pxz + g0.y * pyz + g0.z * pzz);
-        const float ig = rsqrtf(q), ig3 = ig * ig * ig;
-        const float ud = g0.x * F[0].nx + g0.y * F[0].ny + g0.z * F[0].nz;
-        const float dcx = F[0].nx * ig - ud * g0.x * ig3;
-        const float dcy = F[0].ny * ig - ud * g0.y * ig3;
-        const float dcz = F[0].nz * ig - ud * g0.z * ig3;
-        const float cxx = dcx * pxx + dcy * pxy + dcz * pxz;
-        const float cyy = dcx * pxy + dcy * pyy + dcz * pyz;
-        const float czz = dcx * pxz + dcy * pyz + dcz * pzz;
-        const float coef = T[0].coef;
-        // A13_divergence_3d: central differences of da/dphi_p at the neighbours
-        const float ddx = (T[1].da.x - T[2].da.x) * P.half_over_dx;
-        const float ddy = (T[3].da.y - T[4].da.y) * P.half_over_dx;
-        const float ddz = (T[5].da.z - T[6].da.z) * P.half_over_dx;
-        const float a = T[0].a;
-        const float3 d0 = T[0].da;
-        const float Ex = coef * cxx * d0.x * q + a * ddx * q + a * d0.x * qx;
-        const float Ey = coef * cyy * d0.y * q + a * ddy * q + a * d0.y * qy;
-        const float Ez = coef * czz * d0.z * q + a * ddz * q + a * d0.z * qz;
-        lv += P.eps0sq * (Ex + Ey + Ez);
+    for (int p = 1; p < 7; ++p) {
+        const Grad g(P, G[p]);
+        const PointTerms t = point_terms<NT>(P, g, un);
+        const float3 dc = dcos(g, t);
+        const float da = __fmul_rn(t.coef, p < 3 ? dc.x : (p < 5 ? dc.y : dc.z));
+        flux[p] = __fmul_rn(t0.e2 + t.e2, L[p] - L[0]);
+        div[p] = g.valid ? ((p & 1) ? da : -da) : 0.0f;
     }
-    lap_sl = lv;
-    b_sl = calc_b(P, G[0], F[0]);
+    b_sl = 1.0f;
+    center_terms(P, g0, t0, L, st.hxy, st.hxz, st.hyz, arm_sum(flux), arm_sum(div), lap_sl, b_sl);
 }
 
-// Everything of the update of one cell after its active list is known:
-// ids (ascending), values vc and Laplacians lap of the n active phases, the
-// liquid at the 7 points, and the dominant solid ts (index, -1 if none) with
-// its gradient gs.  HEAVY enables the anisotropic solid-liquid terms (cells
-// with liquid and a solid active) with NT normals per grain: 4 where every
-// grain's 8 normals are 4 antipodal pairs (checked on the host), else 8.
-// The per-phase loops are kept rolled, and each kernel is compiled for one
-// NT: unrolled or duplicated copies of this body made the kernels wait on
-// instruction fetch.
-template <int S, int NA, bool HEAVY, int NT>
-__device__ __forceinline__ void update_cell(const In &in, const Out &out, const Mats &M, const Params &P, int l,
-                                            int m, int k, uint32_t c, int n, const int (&ids)[NA],
-                                            const float (&vc)[NA], const float (&lap)[NA], const float (&vL)[7],
-                                            int ts, float3 gs, int32_t *__restrict__ err) {
+// Three forms of the update of a queued cell give the same bits:
+//   pair_cell   one thread, a neighbourhood of the liquid and one solid
+//   trio_cell   one thread, a neighbourhood of up to three phases
+//   octet_cell  eight lanes, any neighbourhood
+// The first two take most cells of a large domain: no per-phase arrays in local
+// memory, and the records in one or two rounds of loads.  What they leave, and
+// everything on small domains, where a step is one cell's latency, goes to the
+// third.  A 256^3 step with 64 grains (0.57 M general cells, 0.30 M pairs, 73 k
+// others, 13 k of them beyond three phases): pairs 29 us, general 28, trios 16,
+// rest 24; with one thread per cell for any neighbourhood, its arrays in local
+// memory, the two list kernels took 150 us.  By octets alone the lists take 292.
+
+// Update of an interface cell whose neighbourhood holds the liquid and one
+// solid (list 1 where the sweep split the lists): no merge, and only the pair's
+// terms.  Returns false, with nothing written, where the neighbourhood holds
+// more.
+template <int NT>
+__device__ __forceinline__ bool pair_cell(const In &in, const Out &out, const Mats &M, const Params &P, int l, int m,
+                                          int k) {
     const uint32_t cells = P.cells32;
-    const int nn = n;
-    const bool has_liq = n > 0 && ids[0] == LIQ;
-    const bool has_solid = n > (has_liq ? 1 : 0);
-    float lap_sl[NA], b_sl[NA];
+    const int lp = wrap_p(l, P.nx), lm = wrap_m(l, P.nx), mp = wrap_p(m, P.ny), mm = wrap_m(m, P.ny);
+    const int kp = clamp_p(k, P.nz), km = clamp_m(k, P.nz);
+    const uint32_t pt[7] = {cidx(P, l, m, k), cidx(P, lp, m, k), cidx(P, lm, m, k), cidx(P, l, mp, k),
+                            cidx(P, l, mm, k), cidx(P, l, m, kp), cidx(P, l, m, km)};
+    uint32_t h[7];
+    float v0[7], v1[7];
+    int i1[7];
+#pragma unroll
+    for (int p = 0; p < 7; ++p) {
+        h[p] = __ldg(in.head + pt[p]);
+        v0[p] = __ldg(in.val + pt[p]);
+        i1[p] = (int)__ldg(in.idx + cells + pt[p]);
+        v1[p] = __ldg(in.val + cells + pt[p]);
+    }
+    float vL[7], vS[7];
+    int sid = 0;
+    bool pair = true;
+#pragma unroll
+    for (int p = 0; p < 7; ++p) {
+        const int n = hcount(h[p]), id = hid0(h[p]);
+        const float v = n >= 2 || hexplicit(h[p]) ? v0[p] : 1.0f;
+        vL[p] = n >= 1 && id == LIQ ? v : 0.0f;
+        vS[p] = n >= 2 ? v1[p] : (n == 1 && id != LIQ ? v : 0.0f);
+        const int s = n >= 2 ? i1[p] : (n == 1 ? id : LIQ);  // the point's solid, LIQ for none
+        pair = pair && (n < 2 || (n == 2 && id == LIQ)) && (s == LIQ || sid == 0 || s == sid);
+        sid = s != LIQ ? s : sid;
+    }
+    if (!pair || sid == 0) return false;
+    const Stencil st(in, P, l, m, k, vL);
+    const float *ug = M.n111 + (size_t)(P.n111_base + sid) * 24;
+    float un[3 * NT], lap_sl, b_sl;
+#pragma unroll
+    for (int q = 0; q < 3 * NT; ++q) un[q] = __ldg(ug + q);
+    interface_terms<NT>(P, st, vL, un, lap_sl, b_sl);
+    const float3 gs = make_float3((vS[1] - vS[2]) * P.inv_2dx, (vS[3] - vS[4]) * P.inv_2dx, (vS[5] - vS[6]) * P.inv_2dx);
+    const float al = point_terms<NT>(P, Grad(P, gs), un).a;
+    const float w_sl = P.w0 * (al * al);
+
+    // the pair (solid, liquid) of trio_cell's sums; (liquid, solid) negates it
+    const int N = P.N;
+    const float WL = fmaf(__ldg(M.wij + sid), vS[0], __fmul_rn(__ldg(M.wij), vL[0]));
+    const float WS = fmaf(__ldg(M.wij + sid * N + sid), vS[0], __fmul_rn(w_sl, vL[0]));
+    const double Tmc = P.clock ? P.clock->tmc[P.parity] : P.Tmc;
+    const float dT = P.t_uniform ? P.dT_uniform : (float)(M.T0z[k] - Tmc);
+    const float ppp = __fadd_rn(__fsub_rn(WS, WL), 0.5f * lap_sl);
+    const float tf = __fmul_rn(__fmul_rn(FORCE_PREF, sqrtf(fmaxf(__fmul_rn(vS[0], vL[0]), 0.0f))), -P.Sf * dT);
+    const float drive = __fsub_rn(ppp, tf);
+    const float mS = __ldg(M.mij + sid * N) * b_sl, mL = __ldg(M.mij + sid) * b_sl;
+    const float dS = -__fmul_rn(__fmul_rn(__fmul_rn(2.0f, mS), 0.5f), drive);
+    const float dL = __fmul_rn(__fmul_rn(__fmul_rn(2.0f, mL), 0.5f), drive);
+    const float oL = fminf(fmaxf(fmaf(P.dt, dL, vL[0]), 0.0f), 1.0f);
+    const float oS = fminf(fmaxf(fmaf(P.dt, dS, vS[0]), 0.0f), 1.0f);
+    // compensated sum of the two, as the loop over phases forms it
+    const float s2 = oL + oS, bb = s2 - oL;
+    const float low = (oL - (s2 - bb)) + (oS - bb);
+    const bool normal = s2 + low > 1e-20f;
+    float inv = 1.0f / s2;
+    inv = fmaf(-__fmul_rn(inv, inv), low, inv);
+    const float rL = normal ? oL * inv : 1.0f, rS = normal ? oS * inv : oS;
+    const uint32_t c = pt[0];
+    const bool keepL = rL > 0.0f, keepS = rS > 0.0f;
+    out.val[c] = keepL ? rL : rS;
+    if (keepL && keepS) {
+        out.idx[cells + c] = (uint16_t)sid;
+        out.val[cells + c] = rS;
+    }
+    out.head[c] = mkhead(keepL || !keepS ? LIQ : sid, (keepL ? 1 : 0) + (keepS ? 1 : 0), false);
+    return true;
+}
+
+// Update of a cell whose neighbourhood holds up to three phases, in registers:
+// HEAVY the multi-solid interface cells (list 2), otherwise list 0 (grain
+// boundaries, and everything of the isotropic model).  Returns false, with
+// nothing written, where the neighbourhood holds more.
+template <int S, bool HEAVY, int NT>
+__device__ __forceinline__ bool trio_cell(const In &in, const Out &out, const Mats &M, const Params &P, int l, int m,
+                                          int k) {
+    constexpr int NONE = 0x7fffffff;
+    const uint32_t cells = P.cells32;
+    const int lp = wrap_p(l, P.nx), lm = wrap_m(l, P.nx), mp = wrap_p(m, P.ny), mm = wrap_m(m, P.ny);
+    const int kp = clamp_p(k, P.nz), km = clamp_m(k, P.nz);
+    const uint32_t pt[7] = {cidx(P, l, m, k), cidx(P, lp, m, k), cidx(P, lm, m, k), cidx(P, l, mp, k),
+                            cidx(P, l, mm, k), cidx(P, l, m, kp), cidx(P, l, m, km)};
+    // each point's list, and its merge by shifting the lists
+    int ia[7], ib[7], ic[7];
+    float va[7], vb[7], vd[7];
+    bool fits = true;
+#pragma unroll
+    for (int p = 0; p < 7; ++p) {
+        const uint32_t h = __ldg(in.head + pt[p]);
+        const float v = __ldg(in.val + pt[p]);
+        const int i1 = (int)__ldg(in.idx + cells + pt[p]);
+        vb[p] = __ldg(in.val + cells + pt[p]);
+        const int n = min(hcount(h), S);
+        ia[p] = n > 0 ? hid0(h) : NONE;
+        va[p] = hcount(h) >= 2 || hexplicit(h) ? v : 1.0f;
+        ib[p] = n > 1 ? i1 : NONE;
+        ic[p] = NONE;
+        vd[p] = 0.0f;
+        if (n > 2) {
+            ic[p] = (int)__ldg(in.idx + 2u * cells + pt[p]);
+            vd[p] = __ldg(in.val + 2u * cells + pt[p]);
+        }
+        fits = fits && n <= 3;
+    }
+    int ids[3];
+    float V[3][7];
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        int id = ia[0];
+#pragma unroll
+        for (int p = 1; p < 7; ++p) id = min(id, ia[p]);
+        ids[t] = id;
+#pragma unroll
+        for (int p = 0; p < 7; ++p) {
+            const bool hit = ia[p] == id && id != NONE;
+            V[t][p] = hit ? va[p] : 0.0f;
+            ia[p] = hit ? ib[p] : ia[p];
+            va[p] = hit ? vb[p] : va[p];
+            ib[p] = hit ? ic[p] : ib[p];
+            vb[p] = hit ? vd[p] : vb[p];
+            ic[p] = hit ? NONE : ic[p];
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < 7; ++p) fits = fits && ia[p] == NONE;
+    if (!fits || ids[0] == NONE) return false;
+    const int n = ids[1] == NONE ? 1 : (ids[2] == NONE ? 2 : 3);
+    float lap[3], lap_sl[3] = {0.0f, 0.0f, 0.0f}, b_sl[3] = {1.0f, 1.0f, 1.0f};
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        lap[t] = lap7(P, V[t]);
+        if (t >= n) ids[t] = LIQ;  // a valid index; never used
+    }
     float w_sl = P.w0;
-    lap_sl[0] = 0.0f;
-    b_sl[0] = 1.0f;
-    if (has_liq && has_solid) {
-        if (HEAVY && P.use_aniso) {
-            const int lp = wrap_p(l, P.nx), lm = wrap_m(l, P.nx), mp = wrap_p(m, P.ny), mm = wrap_m(m, P.ny);
-            const int kp = clamp_p(k, P.nz), km = clamp_m(k, P.nz);
-            // liquid on the 25-point stencil (offsets with |dx|+|dy|+|dz| <= 2)
-            const int lpp = wrap_p(lp, P.nx), lmm = wrap_m(lm, P.nx);
-            const int mpp = wrap_p(mp, P.ny), mmm = wrap_m(mm, P.ny);
-            const int kpp = clamp_p(kp, P.nz), kmm = clamp_m(km, P.nz);
-            const float Lxpyp = liquid32(in, cidx(P, lp, mp, k)), Lxpym = liquid32(in, cidx(P, lp, mm, k));
-            const float Lxmyp = liquid32(in, cidx(P, lm, mp, k)), Lxmym = liquid32(in, cidx(P, lm, mm, k));
-            const float Lxpzp = liquid32(in, cidx(P, lp, m, kp)), Lxpzm = liquid32(in, cidx(P, lp, m, km));
-            const float Lxmzp = liquid32(in, cidx(P, lm, m, kp)), Lxmzm = liquid32(in, cidx(P, lm, m, km));
-            const float Lypzp = liquid32(in, cidx(P, l, mp, kp)), Lypzm = liquid32(in, cidx(P, l, mp, km));
-            const float Lymzp = liquid32(in, cidx(P, l, mm, kp)), Lymzm = liquid32(in, cidx(P, l, mm, km));
-            const float Lx2p = liquid32(in, cidx(P, lpp, m, k)), Lx2m = liquid32(in, cidx(P, lmm, m, k));
-            const float Ly2p = liquid32(in, cidx(P, l, mpp, k)), Ly2m = liquid32(in, cidx(P, l, mmm, k));
-            const float Lz2p = liquid32(in, cidx(P, l, m, kpp)), Lz2m = liquid32(in, cidx(P, l, m, kmm));
-            const float g2 = P.inv_2dx;
-            float3 G[7];
-            G[0] = make_float3((vL[1] - vL[2]) * g2, (vL[3] - vL[4]) * g2, (vL[5] - vL[6]) * g2);
-            G[1] = make_float3((Lx2p - vL[0]) * g2, (Lxpyp - Lxpym) * g2, (Lxpzp - Lxpzm) * g2);
-            G[2] = make_float3((vL[0] - Lx2m) * g2, (Lxmyp - Lxmym) * g2, (Lxmzp - Lxmzm) * g2);
-            G[3] = make_float3((Lxpyp - Lxmyp) * g2, (Ly2p - vL[0]) * g2, (Lypzp - Lypzm) * g2);
-            G[4] = make_float3((Lxpym - Lxmym) * g2, (vL[0] - Ly2m) * g2, (Lymzp - Lymzm) * g2);
-            // z neighbours sit on the clamped rows: at the top/bottom row the
-            // neighbour is the cell itself
-            G[5] = (kp == k) ? G[0] : make_float3((Lxpzp - Lxmzp) * g2, (Lypzp - Lymzp) * g2, (Lz2p - vL[0]) * g2);
-            G[6] = (km == k) ? G[0] : make_float3((Lxpzm - Lxmzm) * g2, (Lypzm - Lymzm) * g2, (vL[0] - Lz2m) * g2);
-            if (kp == k) G[5].z = (vL[5] - vL[6]) * g2;
-            if (km == k) G[6].z = (vL[5] - vL[6]) * g2;
-            float h2[6];
-            const float qq = 0.25f * P.inv_dx2;
-            h2[0] = (vL[1] - 2.0f * vL[0] + vL[2]) * P.inv_dx2;
-            h2[1] = (vL[3] - 2.0f * vL[0] + vL[4]) * P.inv_dx2;
-            h2[2] = (vL[5] - 2.0f * vL[0] + vL[6]) * P.inv_dx2;
-            h2[3] = (Lxpyp - Lxpym - Lxmyp + Lxmym) * qq;
-            h2[4] = (Lxpzp - Lxpzm - Lxmzp + Lxmzm) * qq;
-            h2[5] = (Lypzp - Lypzm - Lymzp + Lymzm) * qq;
+    if (ids[0] == LIQ && n > 1) {
+        if (HEAVY) {
+            const Stencil st(in, P, l, m, k, V[0]);
+            // dominant solid
+            const bool last = n == 3 && V[2][0] > V[1][0];
+            const float3 gs = last ? make_float3((V[2][1] - V[2][2]) * P.inv_2dx, (V[2][3] - V[2][4]) * P.inv_2dx,
+                                                 (V[2][5] - V[2][6]) * P.inv_2dx)
+                                   : make_float3((V[1][1] - V[1][2]) * P.inv_2dx, (V[1][3] - V[1][4]) * P.inv_2dx,
+                                                 (V[1][5] - V[1][6]) * P.inv_2dx);
 #pragma unroll 1
-            for (int t = 1; t < nn; ++t) {
-                const float *ug = M.n111 + (size_t)(P.n111_base + ids[t]) * 24;
-                float un[3 * NT];
+            for (int t = 1; t < n; ++t) {
+                const float *ug = M.n111 + (size_t)(P.n111_base + (t == 1 ? ids[1] : ids[2])) * 24;
+                float un[3 * NT], lv, b;
 #pragma unroll
                 for (int q = 0; q < 3 * NT; ++q) un[q] = __ldg(ug + q);
-                interface_terms<NT>(P, G, vL, h2, un, P.use_torque != 0, lap_sl[t], b_sl[t]);
-            }
-            if (ts > 0) {
-                const Facet fs = facet_n<NT>(gs, M.n111 + (size_t)(P.n111_base + ids[ts]) * 24, P.g2_floor);
-                const float al = calc_a(P, fs.cabs);
-                w_sl = P.w0 * (al * al);
+                interface_terms<NT>(P, st, V[0], un, lv, b);
+                if (t == 1) { lap_sl[1] = lv; b_sl[1] = b; }
+                else { lap_sl[2] = lv; b_sl[2] = b; }
+                if ((t == 2) == last) {
+                    const float al = point_terms<NT>(P, Grad(P, gs), un).a;
+                    w_sl = P.w0 * (al * al);
+                }
             }
         } else {
             // isotropic branch of the switchable kernel (:729-731)
-#pragma unroll 1
-            for (int t = 1; t < nn; ++t) {
-                lap_sl[t] = P.eps0sq * lap[0];
-                b_sl[t] = 1.0f;
-            }
-        }
-    } else {
-#pragma unroll 1
-        for (int t = 1; t < nn; ++t) {
-            lap_sl[t] = 0.0f;
-            b_sl[t] = 1.0f;
+            lap_sl[1] = lap_sl[2] = P.eps0sq * lap[0];
         }
     }
 
@@ -526,127 +543,393 @@ __device__ __forceinline__ void update_cell(const In &in, const Out &out, const 
     // reference splits into W_i - W_j (potential) plus either the
     // solid-liquid term of lap_sl or (A_i - A_j)/2 (gradient energy).
     const int N = P.N;
-    float W[NA], Ag[NA];
-#pragma unroll 1
-    for (int t1 = 0; t1 < nn; ++t1) {
-        const int i = ids[t1];
-        float w = 0.0f, a = 0.0f;
-#pragma unroll 1
-        for (int t3 = 0; t3 < nn; ++t3) {
-            const int q = ids[t3];
-            const float wik = (q == LIQ && i != LIQ) ? w_sl : __ldg(M.wij + i * N + q);
-            w = fmaf(wik, vc[t3], w);
-            a = fmaf(__ldg(M.a2ij + i * N + q), lap[t3], a);
+    float W[3], Ag[3], o[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        W[i] = Ag[i] = o[i] = 0.0f;
+        if (i >= n) continue;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            if (q >= n) continue;
+            const float w = (ids[q] == LIQ && ids[i] != LIQ) ? w_sl : __ldg(M.wij + ids[i] * N + ids[q]);
+            W[i] = fmaf(w, V[q][0], W[i]);
+            Ag[i] = fmaf(__ldg(M.a2ij + ids[i] * N + ids[q]), lap[q], Ag[i]);
         }
-        W[t1] = w;
-        Ag[t1] = a;
+    }
+    const double Tmc = P.clock ? P.clock->tmc[P.parity] : P.Tmc;
+    const float dT = P.t_uniform ? P.dT_uniform : (float)(M.T0z[k] - Tmc);
+    const float inv_n = 1.0f / (float)n;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        if (i >= n) continue;
+        float dpi = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            if (j == i || j >= n) continue;
+            const bool sl = ids[i] != LIQ && ids[j] == LIQ, ls = ids[i] == LIQ && ids[j] != LIQ;
+            const float T = sl ? 0.5f * lap_sl[i] : (ls ? -0.5f * lap_sl[j] : 0.5f * __fsub_rn(Ag[i], Ag[j]));
+            const float ppp = __fadd_rn(__fsub_rn(W[i], W[j]), T);
+            const float df = sl ? -P.Sf * dT : (ls ? P.Sf * dT : 0.0f);
+            const float tf = __fmul_rn(__fmul_rn(FORCE_PREF, sqrtf(fmaxf(__fmul_rn(V[i][0], V[j][0]), 0.0f))), df);
+            float me = __ldg(M.mij + ids[i] * N + ids[j]);
+            if (HEAVY) {
+                if (sl) me *= b_sl[i];
+                else if (ls) me *= b_sl[j];
+            }
+            dpi = __fsub_rn(dpi, __fmul_rn(__fmul_rn(__fmul_rn(2.0f, me), inv_n), __fsub_rn(ppp, tf)));
+        }
+        o[i] = fminf(fmaxf(fmaf(P.dt, dpi, V[i][0]), 0.0f), 1.0f);
+    }
+    // renormalise with a compensated (TwoSum) float accumulation (:663-680)
+    float sum = 0.0f, low = 0.0f;
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        if (t >= n) continue;
+        const float s2 = sum + o[t], bb = s2 - sum;
+        low += (sum - (s2 - bb)) + (o[t] - bb);
+        sum = s2;
+    }
+    const bool normal = sum + low > 1e-20f;
+    float inv = 1.0f / sum;
+    inv = fmaf(-__fmul_rn(inv, inv), low, inv);
+    // stored list: the phases that stay positive, ascending; all clipped to
+    // ~0: the liquid takes the cell (:679-680)
+    const uint32_t c = pt[0];
+    int stored = normal ? 0 : 1, first = LIQ;
+    if (!normal) out.val[c] = 1.0f;
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        const float v = normal ? o[t] * inv : o[t];
+        if (t >= n || !(v > 0.0f) || (!normal && ids[t] == LIQ)) continue;
+        if (stored == 0) first = ids[t];
+        else out.idx[(uint32_t)stored * cells + c] = (uint16_t)ids[t];
+        out.val[(uint32_t)stored * cells + c] = v;
+        ++stored;
+    }
+    // one stored phase: its renormalised value is 1 and is left implicit
+    out.head[c] = mkhead(first, stored, false);
+    return true;
+}
+
+// ---------------------------------------------------------------------------
+// Any queued cell, eight lanes per cell.
+//
+// Lanes 0..6 of an octet stand for the cell and its x+, x-, y+, y-, z+, z-
+// neighbours.  Each loads its own point's records, takes part in the merge of
+// the 7 ascending lists (an octet-wide minimum per phase), loads the three
+// liquid values its gradient needs beyond those the octet holds, and evaluates
+// the facet of every solid at its own point; lane 7 evaluates the dominant
+// solid's facet for w_sl.  After the merge lane t (and t - 8, ...) holds phase t
+// for the pair sums, the renormalisation and the stores.
+//
+// The isotropic model (P.use_aniso 0) and cells without liquid or solid skip
+// the facets.
+// a lane's place in its octet: offsets of its point (d), of the next axis (a)
+struct OctetLane {
+    int p, axis;
+    bool plus;       // on the + side
+    int dl, dm, dk;  // the point's offset from the cell
+    int al, am, ak;  // unit offset along the axis after the point's own
+    __device__ __forceinline__ OctetLane() {
+        p = threadIdx.x & 7;
+        const bool arm = p >= 1 && p <= 6;
+        axis = arm ? (p - 1) >> 1 : 3;
+        plus = (p & 1) != 0;
+        const int s = plus ? 1 : -1;
+        dl = axis == 0 ? s : 0; dm = axis == 1 ? s : 0; dk = axis == 2 ? s : 0;
+        al = axis == 2 ? 1 : 0; am = axis == 0 ? 1 : 0; ak = axis == 1 ? 1 : 0;
+    }
+};
+
+// v of lane src of the octet
+template <typename T>
+__device__ __forceinline__ T from_lane(T v, int src) {
+    return __shfl_sync(0xffffffffu, v, src, 8);
+}
+// phase t of the octet (t the same for the whole warp)
+template <int NH, typename T>
+__device__ __forceinline__ T phase_of(const T (&a)[NH], int t) {
+    T x = a[0];
+#pragma unroll
+    for (int h = 1; h < NH; ++h)
+        if ((t >> 3) == h) x = a[h];
+    return from_lane(x, t & 7);
+}
+
+template <int S, int AMAX, int NT, bool LAST>
+__device__ __forceinline__ bool octet_phases(const In &in, const Out &out, const Mats &M, const Params &P,
+                                           int32_t *__restrict__ err, const OctetLane &O, bool active, int l, int m,
+                                           int k) {
+    constexpr unsigned ALL = 0xffffffffu;
+    constexpr int NH = AMAX / 8;  // phases per lane
+    constexpr int NONE = 0x7fffffff;
+    const uint32_t cells = P.cells32;
+    const int p = O.p, oct = (threadIdx.x & 31) >> 3;
+    auto wrap = [](int a, int n) { return a < 0 ? n - 1 : (a >= n ? 0 : a); };
+    auto clamp = [&](int a) { return min(max(a, 0), P.nz - 1); };
+    const uint32_t c = cidx(P, l, m, k);
+    const int lo = wrap(l + O.dl, P.nx), mo = wrap(m + O.dm, P.ny), ko = clamp(k + O.dk);
+    const uint32_t pt = cidx(P, lo, mo, ko);
+
+    // ---- merge of the 7 lists
+    const uint32_t hw = __ldg(in.head + pt);
+    float cur = __ldg(in.val + pt);
+    // liquid beyond the octet's points: the next point along the lane's axis
+    // and the two beside its own point along the next axis
+    const float L2 = liquid32(in, cidx(P, wrap(lo + O.dl, P.nx), wrap(mo + O.dm, P.ny), clamp(ko + O.dk)));
+    const float LA = liquid32(in, cidx(P, wrap(lo + O.al, P.nx), wrap(mo + O.am, P.ny), clamp(ko + O.ak)));
+    const float LB = liquid32(in, cidx(P, wrap(lo - O.al, P.nx), wrap(mo - O.am, P.ny), clamp(ko - O.ak)));
+    if (!(hcount(hw) >= 2 || hexplicit(hw))) cur = 1.0f;
+    const int cnt = p < 7 ? min(hcount(hw), S) : 0;
+    int next = cnt > 0 ? hid0(hw) : NONE, pos = 0, nid = NONE;
+    float nval = 0.0f;
+    if (cnt >= 2) {
+        nid = (int)__ldg(in.idx + cells + pt);
+        nval = __ldg(in.val + cells + pt);
+    }
+    int ids[NH];
+    float vc[NH], lap[NH];
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+        ids[h] = 0;
+        vc[h] = lap[h] = 0.0f;
+    }
+    int n = 0, ts = -1, first = NONE;
+    bool ovf = false;
+    float vL = 0.0f, maxv = -1.0f;
+    float3 g = make_float3(0.f, 0.f, 0.f);  // gradient of the dominant solid, later of the lane's point
+    while (true) {
+        int id = min(next, __shfl_xor_sync(ALL, next, 1));
+        id = min(id, __shfl_xor_sync(ALL, id, 2));
+        id = min(id, __shfl_xor_sync(ALL, id, 4));
+        const bool live = id != NONE;
+        if (!__any_sync(ALL, live)) break;
+        float own = 0.0f;
+        if (live && next == id) {
+            own = cur;
+            cur = nval;
+            next = nid;
+            ++pos;
+            nid = NONE;
+            if (pos + 1 < cnt) {
+                nid = (int)__ldg(in.idx + (uint32_t)(pos + 1) * cells + pt);
+                nval = __ldg(in.val + (uint32_t)(pos + 1) * cells + pt);
+            }
+        }
+        const float v[7] = {from_lane(own, 0), from_lane(own, 1), from_lane(own, 2), from_lane(own, 3), from_lane(own, 4), from_lane(own, 5), from_lane(own, 6)};
+        if (live && n == AMAX) {
+            ovf = true;
+            next = NONE;
+        } else if (live) {
+            if (n == 0) first = id;
+#pragma unroll
+            for (int h = 0; h < NH; ++h)
+                if (n == 8 * h + p) {
+                    ids[h] = id;
+                    vc[h] = v[0];
+                    lap[h] = lap7(P, v);
+                }
+            if (id == LIQ) {
+                vL = own;
+            } else if (v[0] > maxv) {
+                maxv = v[0];
+                ts = n;
+                g = make_float3((v[1] - v[2]) * P.inv_2dx, (v[3] - v[4]) * P.inv_2dx, (v[5] - v[6]) * P.inv_2dx);
+            }
+            ++n;
+        }
+    }
+    if (!LAST && __any_sync(ALL, ovf)) return false;
+    const int n_most = __reduce_max_sync(ALL, n);
+
+    // ---- solid-liquid terms
+    float lap_sl[NH], b_sl[NH];
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+        lap_sl[h] = 0.0f;
+        b_sl[h] = 1.0f;
+    }
+    const bool heavy = n > 1 && first == LIQ;  // solids beside liquid
+    float w_sl = P.w0;
+    if (!P.use_aniso) {
+        // isotropic branch of the switchable kernel (:729-731)
+        const float lap_liq = from_lane(lap[0], 0);
+#pragma unroll
+        for (int h = 0; h < NH; ++h)
+            if (heavy) lap_sl[h] = P.eps0sq * lap_liq;
+    } else if (__any_sync(ALL, heavy)) {
+        const float L[7] = {from_lane(vL, 0), from_lane(vL, 1), from_lane(vL, 2), from_lane(vL, 3), from_lane(vL, 4), from_lane(vL, 5), from_lane(vL, 6)};
+        // the point's gradient: along its own axis, the next one, the third
+        float along = O.plus ? L2 - L[0] : L[0] - L2;
+        // a z neighbour beyond the domain is the cell itself
+        if (O.axis == 2 && ko == k) along = L[5] - L[6];
+        const float beside = LA - LB;
+        const int q0 = O.axis == 0 ? 5 : (O.axis == 1 ? 1 : 3);
+        const float Ap = from_lane(LA, q0), Am = from_lane(LA, q0 + 1), Bp = from_lane(LB, q0), Bm = from_lane(LB, q0 + 1);
+        const float across = O.plus ? Ap - Am : Bp - Bm;
+        const float hxy = from_lane(beside, 1) - from_lane(beside, 2), hxz = from_lane(across, 1) - from_lane(across, 2);
+        const float hyz = from_lane(beside, 3) - from_lane(beside, 4);
+        const float3 g0 = make_float3((L[1] - L[2]) * P.inv_2dx, (L[3] - L[4]) * P.inv_2dx, (L[5] - L[6]) * P.inv_2dx);
+        if (O.axis < 3) {
+            const float u = along * P.inv_2dx, v = beside * P.inv_2dx, w = across * P.inv_2dx;
+            g = O.axis == 0 ? make_float3(u, v, w) : (O.axis == 1 ? make_float3(w, u, v) : make_float3(v, w, u));
+        } else if (p == 0) {
+            g = g0;
+        }
+        const Grad G(P, g);
+        const bool any = (__ballot_sync(ALL, G.valid && p < 7) >> (8 * oct) & 0x7fu) != 0u;
+        const float dL = vL - L[0];
+        float al = 0.0f;
+#pragma unroll 1
+        for (int t = 1; t < n_most; ++t) {
+            const bool solid = heavy && t < n;
+            const int id = phase_of(ids, t);
+            const float *u = M.n111 + (size_t)(P.n111_base + (solid ? id : 0)) * 24;
+            float un[3 * NT];
+#pragma unroll
+            for (int i = 0; i < 3 * NT; ++i) un[i] = __ldg(u + i);
+            const PointTerms T = point_terms<NT>(P, G, un);
+            if (t == ts) al = T.a;  // used from lane 7
+            const float3 dc = dcos(G, T);
+            const float e2_0 = from_lane(T.e2, 0);
+            const float da = __fmul_rn(T.coef, O.axis == 0 ? dc.x : (O.axis == 1 ? dc.y : dc.z));
+            // sums over the six arms (arm_sum's order)
+            float flux = O.axis < 3 ? __fmul_rn(e2_0 + T.e2, dL) : 0.0f;
+            float div = O.axis < 3 && G.valid ? (O.plus ? da : -da) : 0.0f;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                flux = __fadd_rn(flux, __shfl_xor_sync(ALL, flux, o));
+                div = __fadd_rn(div, __shfl_xor_sync(ALL, div, o));
+            }
+            float lv = 0.0f, b = any ? 1.0f : P.b_flat;
+            if (p == 0 && solid) center_terms(P, G, T, L, hxy, hxz, hyz, flux, div, lv, b);
+            __syncwarp();
+            lv = from_lane(lv, 0);
+            b = from_lane(b, 0);
+#pragma unroll
+            for (int h = 0; h < NH; ++h)
+                if (solid && t == 8 * h + p) {
+                    lap_sl[h] = lv;
+                    b_sl[h] = b;
+                }
+        }
+        al = from_lane(al, 7);
+        if (heavy && ts > 0) w_sl = P.w0 * (al * al);
+    }
+
+    // ---- pair sums (trio_cell), lane t on phase t
+    const int N = P.N;
+    float W[NH], Ag[NH], dpi[NH], outv[NH];
+#pragma unroll
+    for (int h = 0; h < NH; ++h) W[h] = Ag[h] = dpi[h] = outv[h] = 0.0f;
+    // (no branch on t < n: the loads of two phases are in flight together)
+#pragma unroll 2
+    for (int t = 0; t < n_most; ++t) {
+        const int id = phase_of(ids, t);
+        const float v = phase_of(vc, t), lp = phase_of(lap, t);
+        const bool has = t < n;
+#pragma unroll
+        for (int h = 0; h < NH; ++h) {
+            if (h > 0 && 8 * h >= n_most) break;
+            const float w0 = __ldg(M.wij + ids[h] * N + id), a2 = __ldg(M.a2ij + ids[h] * N + id);
+            const float w = (id == LIQ && ids[h] != LIQ) ? w_sl : w0;
+            W[h] = has ? fmaf(w, v, W[h]) : W[h];
+            Ag[h] = has ? fmaf(a2, lp, Ag[h]) : Ag[h];
+        }
     }
     const double Tmc = P.clock ? P.clock->tmc[P.parity] : P.Tmc;
     const float dT = P.t_uniform ? P.dT_uniform : (float)(M.T0z[k] - Tmc);
     const float inv_n = 1.0f / (float)(n > 0 ? n : 1);
-    // the non-heavy build: lap_sl is eps0^2 times the liquid's Laplacian for
-    // every solid (the isotropic branch above) and b_sl is 1, so its arrays
-    // stay out of local memory
-    const float lsl_iso = (has_liq && has_solid) ? P.eps0sq * lap[0] : 0.0f;
-    float outv[NA];
-#pragma unroll 1
-    for (int t1 = 0; t1 < nn; ++t1) {
-        const int i = ids[t1];
-        float dpi = 0.0f;
-#pragma unroll 1
-        for (int t2 = 0; t2 < nn; ++t2) {
-            if (t2 == t1) continue;
-            const int j = ids[t2];
+#pragma unroll 2
+    for (int t = 0; t < n_most; ++t) {
+        const int j = phase_of(ids, t);
+        const float v2 = phase_of(vc, t), W2 = phase_of(W, t), A2 = phase_of(Ag, t), l2 = phase_of(lap_sl, t), b2 = phase_of(b_sl, t);
+#pragma unroll
+        for (int h = 0; h < NH; ++h) {
+            if (h > 0 && 8 * h >= n_most) break;
+            const bool has = t < n && t != 8 * h + p;
+            const int i = ids[h];
             const bool sl = (i != LIQ && j == LIQ), ls = (i == LIQ && j != LIQ);
-            const float L1 = HEAVY ? lap_sl[t1] : lsl_iso, L2 = HEAVY ? lap_sl[t2] : lsl_iso;
-            const float T = sl ? 0.5f * L1 : (ls ? -0.5f * L2 : 0.5f * __fsub_rn(Ag[t1], Ag[t2]));
-            const float ppp = __fadd_rn(__fsub_rn(W[t1], W[t2]), T);
-            const float df = sl ? -P.Sf * dT : (ls ? P.Sf * dT : 0.0f);
-            const float tf = __fmul_rn(__fmul_rn(FORCE_PREF, sqrtf(fmaxf(__fmul_rn(vc[t1], vc[t2]), 0.0f))), df);
             float me = __ldg(M.mij + i * N + j);
-            if (HEAVY) {
-                if (sl) me *= b_sl[t1];
-                else if (ls) me *= b_sl[t2];
-            }
-            dpi = __fsub_rn(dpi, __fmul_rn(__fmul_rn(__fmul_rn(2.0f, me), inv_n), __fsub_rn(ppp, tf)));
+            const float T = sl ? 0.5f * lap_sl[h] : (ls ? -0.5f * l2 : 0.5f * __fsub_rn(Ag[h], A2));
+            const float ppp = __fadd_rn(__fsub_rn(W[h], W2), T);
+            const float df = sl ? -P.Sf * dT : (ls ? P.Sf * dT : 0.0f);
+            const float tf = __fmul_rn(__fmul_rn(FORCE_PREF, sqrtf(fmaxf(__fmul_rn(vc[h], v2), 0.0f))), df);
+            me = sl ? me * b_sl[h] : (ls ? me * b2 : me);
+            const float d = __fsub_rn(dpi[h], __fmul_rn(__fmul_rn(__fmul_rn(2.0f, me), inv_n), __fsub_rn(ppp, tf)));
+            dpi[h] = has ? d : dpi[h];
         }
-        outv[t1] = fminf(fmaxf(fmaf(P.dt, dpi, vc[t1]), 0.0f), 1.0f);
     }
-
+#pragma unroll
+    for (int h = 0; h < NH; ++h)
+        if (8 * h + p < n) outv[h] = fminf(fmaxf(fmaf(P.dt, dpi[h], vc[h]), 0.0f), 1.0f);
     // renormalise with a compensated (TwoSum) float accumulation (:663-680)
-    float sh = 0.0f, sl_ = 0.0f;
+    float sum = 0.0f, low = 0.0f;
 #pragma unroll 1
-    for (int t = 0; t < nn; ++t) {
-        const float a = sh, b = outv[t];
-        const float s2 = a + b;
-        const float bb = s2 - a;
-        sl_ += (a - (s2 - bb)) + (b - bb);
-        sh = s2;
+    for (int t = 0; t < n_most; ++t) {
+        const float b = phase_of(outv, t);
+        const float s2 = sum + b;
+        const float bb = s2 - sum;
+        low = t < n ? low + ((sum - (s2 - bb)) + (b - bb)) : low;
+        sum = t < n ? s2 : sum;
     }
-    // stored list: the phases that stay positive, ascending
-    int cnt_out = 0, id_first = LIQ;
-    bool sovf = false;
-    const bool normal = sh + sl_ > 1e-20f;
-    float inv = 1.0f / sh;
-    inv = fmaf(-__fmul_rn(inv, inv), sl_, inv);
-    if (!normal) {
-        // all clipped to ~0: the liquid takes the cell (:679-680)
-        out.val[c] = 1.0f;
-        id_first = LIQ;
-        cnt_out = 1;
+    // stored list: the phases that stay positive, ascending; all clipped to
+    // ~0: the liquid takes the cell (:679-680)
+    const bool normal = sum + low > 1e-20f;
+    float inv = 1.0f / sum;
+    inv = fmaf(-__fmul_rn(inv, inv), low, inv);
+    int stored = normal ? 0 : 1, id_first = LIQ;
+    const bool writes = active && !ovf;
+#pragma unroll
+    for (int h = 0; h < NH; ++h) {
+        const float v = normal ? outv[h] * inv : outv[h];
+        const bool keep = 8 * h + p < n && v > 0.0f && (normal || ids[h] != LIQ);
+        const uint32_t mask = __ballot_sync(ALL, keep) >> (8 * oct) & 0xffu;
+        const int at = stored + __popc(mask & ((1u << p) - 1u));
+        const int id = from_lane(ids[h], max(__ffs(mask) - 1, 0));
+        if (stored == 0 && mask) id_first = id;
+        if (writes && keep && at < S) {
+            if (at > 0) out.idx[(uint32_t)at * cells + c] = (uint16_t)ids[h];
+            out.val[(uint32_t)at * cells + c] = v;
+        }
+        stored += __popc(mask);
     }
-#pragma unroll 1
-    for (int t = 0; t < nn; ++t) {
-        float v;
-        if (normal) {
-            v = outv[t] * inv;
+    if (p == 0 && active) {
+        if (ovf) {
+            // leave the cell as it was and report; the host re-runs the step
+            // with a wider template
+            atomicOr(err, MPF3D_DEV_SLOT_OVERFLOW);
+            const int c0 = min(hcount(hw), S);
+            out.head[c] = hw;
+            for (int s = 0; s < c0; ++s) {
+                out.idx[(uint32_t)s * cells + c] = __ldg(in.idx + (uint32_t)s * cells + c);
+                out.val[(uint32_t)s * cells + c] = __ldg(in.val + (uint32_t)s * cells + c);
+            }
         } else {
-            if (ids[t] == LIQ) continue;
-            v = outv[t];
+            if (!normal) out.val[c] = 1.0f;
+            // one stored phase: its renormalised value is 1 and is left implicit
+            out.head[c] = mkhead(id_first, min(stored, S), false);
+            if (stored > S) atomicOr(err, MPF3D_DEV_SLOT_OVERFLOW);
         }
-        if (!(v > 0.0f)) continue;
-        if (cnt_out == S) {
-            sovf = true;
-            continue;
-        }
-        if (cnt_out == 0) id_first = ids[t];
-        else out.idx[(uint32_t)cnt_out * cells + c] = (uint16_t)ids[t];
-        out.val[(uint32_t)cnt_out * cells + c] = v;
-        ++cnt_out;
     }
-    // one stored phase: its renormalised value is 1 and is left implicit
-    out.head[c] = mkhead(id_first, cnt_out, false);
-    if (sovf) atomicOr(err, MPF3D_DEV_SLOT_OVERFLOW);
+    return true;
 }
 
-// Update of one cell whose neighbourhood is not uniform: the 7-way merge of
-// the neighbour lists, then update_cell over up to AMAX active phases (NT:
-// normals per grain, used by the HEAVY form only).
-template <int S, int AMAX, bool HEAVY, int NT = 4>
-__device__ __forceinline__ void process_cell(const In &in, const Out &out, const Mats &M, const Params &P,
-                                             int32_t *__restrict__ err, int l, int m, int k) {
-    const uint32_t cells = P.cells32;
-    const int lp = wrap_p(l, P.nx), lm = wrap_m(l, P.nx), mp = wrap_p(m, P.ny), mm = wrap_m(m, P.ny);
-    const int kp = clamp_p(k, P.nz), km = clamp_m(k, P.nz);
-    const uint32_t pt[7] = {cidx(P, l, m, k), cidx(P, lp, m, k), cidx(P, lm, m, k), cidx(P, l, mp, k),
-                            cidx(P, l, mm, k), cidx(P, l, m, kp), cidx(P, l, m, km)};
-    const uint32_t c = pt[0];
-    Active<AMAX> A;
-    gather<S, AMAX>(in, P, pt, A);
-    if (A.ovf) {
-        // leave the cell as it was and report; the host re-runs the step with
-        // a wider template
-        atomicOr(err, MPF3D_DEV_SLOT_OVERFLOW);
-        const uint32_t h0 = __ldg(in.head + c);
-        const int c0 = min(hcount(h0), S);
-        out.head[c] = h0;
-        for (int s = 0; s < c0; ++s) {
-            out.idx[(uint32_t)s * cells + c] = __ldg(in.idx + (uint32_t)s * cells + c);
-            out.val[(uint32_t)s * cells + c] = __ldg(in.val + (uint32_t)s * cells + c);
-        }
-        return;
-    }
-    update_cell<S, AMAX, HEAVY, NT>(in, out, M, P, l, m, k, c, A.n, A.ids, A.vc, A.lap, A.vL, A.ts, A.gs, err);
+// the cells of a warp by up to 8 phases, one per lane; where one has more, by
+// AMAX (out of line: its arrays would cost the common case registers)
+template <int S, int AMAX, int NT>
+__device__ __forceinline__ void octet_many(const In &in, const Out &out, const Mats &M, const Params &P,
+                                        int32_t *__restrict__ err, const OctetLane &O, bool active, int l, int m,
+                                        int k) {
+    octet_phases<S, AMAX, NT, true>(in, out, M, P, err, O, active, l, m, k);
+}
+
+template <int S, int AMAX, int NT>
+__device__ __forceinline__ void octet_cell(const In &in, const Out &out, const Mats &M, const Params &P,
+                                           int32_t *__restrict__ err, const OctetLane &O, bool active, int l, int m,
+                                           int k) {
+    if (!octet_phases<S, 8, NT, AMAX == 8>(in, out, M, P, err, O, active, l, m, k))
+        octet_many<S, AMAX, NT>(in, out, M, P, err, O, active, l, m, k);
 }
 
 // Kernel 1 of a step: every cell.  Uniform neighbourhoods (the cell and its
@@ -714,8 +997,9 @@ struct BlockSink {
 // beyond the domain is the cell itself): a uniform neighbourhood is written
 // directly; any other cell goes to a work list.  Returns whether uniform.
 template <class Sink>
-__device__ __forceinline__ bool sweep_cell(const Out &out, const Params &P, bool split, Sink &sink, int j, uint32_t c,
-                                           uint32_t h0, const uint32_t (&hn)[6]) {
+__device__ __forceinline__ bool sweep_cell(const In &in, const Out &out, const Params &P, bool split, Sink &sink,
+                                           int j, uint32_t c, uint32_t h0, const uint32_t (&hn)[6],
+                                           const uint32_t (&qn)[6]) {
     bool uniform = hcount(h0) == 1 && !hexplicit(h0);
 #pragma unroll
     for (int p = 0; p < 6; ++p) uniform = uniform && hn[p] == h0;
@@ -736,9 +1020,11 @@ __device__ __forceinline__ bool sweep_cell(const Out &out, const Params &P, bool
     bool multi = false;
     if (heavy && split) {
         // several solids in the active list: a head with 3+ phases or two
-        // solids, or two different solid first ids
+        // solids, two different solid first ids, or -- read only where the
+        // heads do not tell -- different solids beside the liquid
         int sid = -1;
         const uint32_t hs[7] = {h0, hn[0], hn[1], hn[2], hn[3], hn[4], hn[5]};
+        const uint32_t qs[7] = {c, qn[0], qn[1], qn[2], qn[3], qn[4], qn[5]};
 #pragma unroll
         for (int p = 0; p < 7; ++p) {
             const int cn = hcount(hs[p]), id = hid0(hs[p]);
@@ -746,6 +1032,18 @@ __device__ __forceinline__ bool sweep_cell(const Out &out, const Params &P, bool
             else if (cn >= 1 && id != LIQ) {
                 if (sid < 0) sid = id;
                 else if (sid != id) multi = true;
+            }
+        }
+        if (!multi) {
+            int second[7];
+#pragma unroll
+            for (int p = 0; p < 7; ++p)
+                second[p] = hcount(hs[p]) == 2 ? (int)__ldg(in.idx + P.cells32 + qs[p]) : -1;
+#pragma unroll
+            for (int p = 0; p < 7; ++p) {
+                if (second[p] < 0) continue;
+                if (sid < 0) sid = second[p];
+                else if (sid != second[p]) multi = true;
             }
         }
     }
@@ -787,7 +1085,8 @@ __device__ __forceinline__ bool sweep_column(const In &in, const Out &out, const
         // a z neighbour beyond the domain is the cell itself (clamped index)
         if (k == P.nz - 1) hn[4] = h0;
         if (k == 0) hn[5] = h0;
-        all_uniform = sweep_cell(out, P, split, sink, j, c, h0, hn) && all_uniform;
+        const uint32_t qn[6] = {qxp, qxm, qyp, qym, k < P.nz - 1 ? c + plane : c, k > 0 ? c - plane : c};
+        all_uniform = sweep_cell(in, out, P, split, sink, j, c, h0, hn, qn) && all_uniform;
     }
     return all_uniform;
 }
@@ -799,8 +1098,9 @@ __device__ __forceinline__ bool sweep_column(const In &in, const Out &out, const
 constexpr int TMA_X = 40;
 
 template <int ZB, class Sink>
-__device__ __forceinline__ bool sweep_column_tile(const uint32_t *tile, int rows, const Out &out, const Params &P,
-                                                  bool split, Sink &sink, int l, int m, int k0, int l0, int m0) {
+__device__ __forceinline__ bool sweep_column_tile(const uint32_t *tile, int rows, const In &in, const Out &out,
+                                                  const Params &P, bool split, Sink &sink, int l, int m, int k0,
+                                                  int l0, int m0) {
     const uint32_t plane = (uint32_t)P.nx * (uint32_t)P.ny;
     const uint32_t col = (uint32_t)m * (uint32_t)P.nx + (uint32_t)l;
     const int xi = l - l0 + 4, yi = m - m0 + 1;
@@ -817,7 +1117,13 @@ __device__ __forceinline__ bool sweep_column_tile(const uint32_t *tile, int rows
                           at(xi, yi - 1, zi), at(xi, yi, zi + 1), at(xi, yi, zi - 1)};
         if (k == P.nz - 1) hn[4] = h0;
         if (k == 0) hn[5] = h0;
-        all_uniform = sweep_cell(out, P, split, sink, j, c, h0, hn) && all_uniform;
+        const uint32_t row = (uint32_t)k * plane;
+        const uint32_t qn[6] = {row + (uint32_t)m * (uint32_t)P.nx + (uint32_t)wrap_p(l, P.nx),
+                                row + (uint32_t)m * (uint32_t)P.nx + (uint32_t)wrap_m(l, P.nx),
+                                row + (uint32_t)wrap_p(m, P.ny) * (uint32_t)P.nx + (uint32_t)l,
+                                row + (uint32_t)wrap_m(m, P.ny) * (uint32_t)P.nx + (uint32_t)l,
+                                k < P.nz - 1 ? c + plane : c, k > 0 ? c - plane : c};
+        all_uniform = sweep_cell(in, out, P, split, sink, j, c, h0, hn, qn) && all_uniform;
     }
     return all_uniform;
 }
@@ -1050,11 +1356,11 @@ __global__ void __launch_bounds__(512, 3) sweep_kernel_tma(const __grid_constant
     BlockSink<ZB> sink(s_cnt);
     if (row_ok && staged) {
         if (!T.flags) {
-            if (l < P.nx) sweep_column_tile<ZB>(tile, rows, out, P, Q.split, sink, l, m, k0, l0, m0);
+            if (l < P.nx) sweep_column_tile<ZB>(tile, rows, in, out, P, Q.split, sink, l, m, k0, l0, m0);
         } else if (quiet) {
             if (threadIdx.x == 0) fout[t] = 1;
         } else {
-            const bool uni = l < P.nx ? sweep_column_tile<ZB>(tile, rows, out, P, Q.split, sink, l, m, k0, l0, m0)
+            const bool uni = l < P.nx ? sweep_column_tile<ZB>(tile, rows, in, out, P, Q.split, sink, l, m, k0, l0, m0)
                                       : true;
             const bool all = __all_sync(0xffffffffu, uni);
             if (threadIdx.x == 0) fout[t] = all ? 1 : 0;
@@ -1074,41 +1380,164 @@ __global__ void __launch_bounds__(512, 3) sweep_kernel_tma(const __grid_constant
                    k0);
 }
 
-// Kernel 2 of a step: the cells queued for the general update, one thread
-// per cell.  Capped at 48 registers (5 blocks of 256 per SM): it waits on
-// memory, and more resident warps beat the few spilled values.
-template <int S, int AMAX>
-__global__ void __launch_bounds__(256, 5) general_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity,
-                                                     int32_t *__restrict__ err) {
-    const uint32_t n = *(volatile uint32_t *)(Q.count + 2 * parity);
-    const uint32_t plane = (uint32_t)P.nx * (uint32_t)P.ny;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t c = Q.items[i];
-        const int k = (int)(c / plane);
-        const uint32_t r = c - (uint32_t)k * plane;
-        const int m = (int)(r / (uint32_t)P.nx);
-        const int l = (int)(r - (uint32_t)m * (uint32_t)P.nx);
-        process_cell<S, AMAX, false>(in, out, M, P, err, l, m, k);
+// The work lists: 0 at items[0..), 1 at items[cells-1..] downwards, 2 at
+// items[cells..).
+struct Lists {
+    uint32_t n[3];
+    __device__ __forceinline__ Lists(const Queue &Q, int parity) {
+        n[0] = *(volatile uint32_t *)(Q.count + 2 * parity);
+        n[1] = *(volatile uint32_t *)(Q.count + 2 * parity + 1);
+        n[2] = Q.split ? *(volatile uint32_t *)(Q.count + 4 + parity) : 0u;
+    }
+    // index in items of entry i of the lists one after the other
+    __device__ __forceinline__ uint32_t item(uint32_t i, uint32_t cells) const {
+        if (i < n[0]) return i;
+        i -= n[0];
+        return i < n[1] ? cells - 1u - i : cells + (i - n[1]);
+    }
+};
+
+// calls cell(c, active) for the cells of all lists, four per warp and call
+template <class Cell>
+__device__ __forceinline__ void for_octets(const Queue &Q, uint32_t cells, int parity, Cell &&cell) {
+    const Lists L(Q, parity);
+    const uint32_t n = L.n[0] + L.n[1] + L.n[2], oct = (threadIdx.x & 31u) >> 3;
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    for (uint32_t w = warp; w * 4u < n; w += warps) {
+        const uint32_t i = w * 4u + oct;
+        cell(Q.items[L.item(min(i, n - 1u), cells)], i < n);
     }
 }
 
-// Kernel 3 of a step: the queued solid-liquid interface cells, one thread
-// per cell, all lanes of a warp on the same (heavy) path; NT normals per
+// Items get(0..n) one per thread, by take(item); those it refuses by
+// rest(item, active), eight lanes each, shared out over the block's warps: they
+// lie in clusters, and a warp that kept its own would take several, at 8-10 us
+// each, one after the other.  For the same reason a block takes runs of RUN
+// items from distant parts of the range; PER: items that make another block
+// worth starting.
+constexpr uint32_t LEFT_CELLS = 1024;
+
+template <uint32_t RUN, uint32_t PER, class Get, class Take, class Rest>
+__device__ __forceinline__ void for_items(uint32_t n, Get &&get, Take &&take, Rest &&rest) {
+    __shared__ uint32_t left[LEFT_CELLS], n_left;
+    const uint32_t blocks = min(gridDim.x, (n + PER - 1u) / PER);
+    if (blockIdx.x >= blocks) return;
+    const uint32_t warp = threadIdx.x >> 5, oct = (threadIdx.x & 31u) >> 3;
+    const uint32_t step = blocks * blockDim.x, passes = LEFT_CELLS / blockDim.x;
+    if (threadIdx.x == 0) n_left = 0;
+    __syncthreads();
+    for (uint32_t at0 = 0; at0 < n;) {
+        for (uint32_t pass = 0; pass < passes && at0 < n; ++pass, at0 += step) {
+            const uint32_t i = at0 + (threadIdx.x / RUN * blocks + blockIdx.x) * RUN + threadIdx.x % RUN;
+            if (i >= n) continue;
+            const uint32_t c = get(i);
+            if (!take(c)) left[atomicAdd(&n_left, 1u)] = c;
+        }
+        __syncthreads();
+        const uint32_t m = n_left;
+        for (uint32_t w = warp; w * 4u < m; w += blockDim.x >> 5)
+            rest(left[min(w * 4u + oct, m - 1u)], w * 4u + oct < m);
+        __syncthreads();
+        if (threadIdx.x == 0) n_left = 0;
+        __syncthreads();
+    }
+}
+
+// Set in the items that trio_cell left to the octets of a kernel of their own
+// (lists 0 and 2; list 1 instead of 2 where the sweep kept all interface cells
+// there).
+constexpr uint32_t LEFT = 0x80000000u;
+
+struct Place {
+    int l, m, k;
+    __device__ __forceinline__ Place(uint32_t r0, int nx, int ny) {
+        const uint32_t plane = (uint32_t)nx * (uint32_t)ny;
+        k = (int)(r0 / plane);
+        const uint32_t r = r0 - (uint32_t)k * plane;
+        m = (int)(r / (uint32_t)nx);
+        l = (int)(r - (uint32_t)m * (uint32_t)nx);
+    }
+};
+
+// Kernel 2 of a step on small domains: eight lanes per cell.  NT: normals per
 // grain (4 or 8, from P.sym_normals).
 template <int S, int AMAX, int NT>
-__global__ void __launch_bounds__(128, 5) interface_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity,
-                                                           int32_t *__restrict__ err) {
-    const uint32_t na = *(volatile uint32_t *)(Q.count + 2 * parity + 1);
-    const uint32_t n = na + (Q.split ? *(volatile uint32_t *)(Q.count + 4 + parity) : 0u);
-    const uint32_t plane = (uint32_t)P.nx * (uint32_t)P.ny;
+__global__ void __launch_bounds__(128, 8) octet_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity,
+                                                       int32_t *__restrict__ err) {
+    const OctetLane O;
+    for_octets(Q, P.cells32, parity, [&](uint32_t c, bool active) {
+        const Place at(c, P.nx, P.ny);
+        octet_cell<S, AMAX, NT>(in, out, M, P, err, O, active, at.l, at.m, at.k);
+    });
+}
+
+// The work-list kernels on large domains: list 1 by pair_cell, where the sweep
+// kept it to pairs, beside lists 2 and 0 by trio_cell.
+template <int NT>
+__global__ void __launch_bounds__(128, 5) pair_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity) {
+    const uint32_t n = *(volatile uint32_t *)(Q.count + 2 * parity + 1);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t c = i < na ? Q.items[P.cells32 - 1u - i] : Q.items[P.cells32 + (i - na)];
-        const int k = (int)(c / plane);
-        const uint32_t r = c - (uint32_t)k * plane;
-        const int m = (int)(r / (uint32_t)P.nx);
-        const int l = (int)(r - (uint32_t)m * (uint32_t)P.nx);
-        process_cell<S, AMAX, true, NT>(in, out, M, P, err, l, m, k);
+        const Place at(Q.items[P.cells32 - 1u - i], P.nx, P.ny);
+        pair_cell<NT>(in, out, M, P, at.l, at.m, at.k);
     }
+}
+
+// list 2: multi-solid interface cells
+template <int S, int NT>
+__global__ void __launch_bounds__(128, 4) trio_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity) {
+    const uint32_t n = *(volatile uint32_t *)(Q.count + (Q.split ? 4 + parity : 2 * parity + 1));
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        uint32_t &item = Q.items[Q.split ? P.cells32 + i : P.cells32 - 1u - i];
+        const uint32_t c = item;
+        const Place at(c, P.nx, P.ny);
+        if (!trio_cell<S, true, NT>(in, out, M, P, at.l, at.m, at.k)) item = c | LEFT;
+    }
+}
+
+// list 0: grain boundaries and junctions, beside the above
+template <int S>
+__global__ void __launch_bounds__(256, 3) general_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity) {
+    const uint32_t n = *(volatile uint32_t *)(Q.count + 2 * parity);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t c = Q.items[i];
+        const Place at(c, P.nx, P.ny);
+        if (!trio_cell<S, false, 4>(in, out, M, P, at.l, at.m, at.k)) Q.items[i] = c | LEFT;
+    }
+}
+
+// what the two left
+template <int S, int AMAX, int NT>
+__global__ void __launch_bounds__(128, 8)
+    rest_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity, int32_t *__restrict__ err) {
+    const OctetLane O;
+    Lists L(Q, parity);
+    if (Q.split) L.n[1] = 0;
+    for_items<8, 32>(
+        L.n[0] + L.n[1] + L.n[2], [&](uint32_t i) { return Q.items[L.item(i, P.cells32)]; },
+        [](uint32_t c) { return (c & LEFT) == 0u; },
+        [&](uint32_t marked, bool active) {
+            const uint32_t c = marked & ~LEFT;
+            const Place at(c, P.nx, P.ny);
+            octet_cell<S, AMAX, NT>(in, out, M, P, err, O, active, at.l, at.m, at.k);
+        });
+}
+
+// list 0 of the isotropic model, which has no other: what trio_cell leaves is
+// done by the same block
+template <int S, int AMAX>
+__global__ void __launch_bounds__(256, 3)
+    isotropic_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity, int32_t *__restrict__ err) {
+    const OctetLane O;
+    for_items<32, 256>(
+        *(volatile uint32_t *)(Q.count + 2 * parity), [&](uint32_t i) { return Q.items[i]; },
+        [&](uint32_t c) {
+            const Place at(c, P.nx, P.ny);
+            return trio_cell<S, false, 4>(in, out, M, P, at.l, at.m, at.k);
+        },
+        [&](uint32_t c, bool active) {
+            const Place at(c, P.nx, P.ny);
+            octet_cell<S, AMAX, 4>(in, out, M, P, err, O, active, at.l, at.m, at.k);
+        });
 }
 
 // ---------------------------------------------------------------------------
@@ -1288,25 +1717,94 @@ __global__ void __launch_bounds__(256) batched_sweep_kernel(In in, Out out, Para
                    P.base + (uint32_t)m * (uint32_t)P.nx + (uint32_t)l, k0);
 }
 
-template <int S, int AMAX, bool HEAVY, int NT = 4>
-__global__ void __launch_bounds__(HEAVY ? 128 : 256) batched_queue_kernel(In in, Out out, Mats M, Params P0,
-                                                                          const mpf3d_instance *__restrict__ inst,
-                                                                          int n_inst, Queue Q, int parity,
-                                                                          int32_t *__restrict__ err) {
-    const uint32_t na = *(volatile uint32_t *)(Q.count + 2 * parity + (HEAVY ? 1 : 0));
-    const uint32_t n = na + ((HEAVY && Q.split) ? *(volatile uint32_t *)(Q.count + 4 + parity) : 0u);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t c = !HEAVY ? Q.items[i] : (i < na ? Q.items[P0.cells32 - 1u - i] : Q.items[P0.cells32 + (i - na)]);
+// The work-list kernels of a batch: as the single domain's, on the instance of
+// each cell.
+template <int S, int AMAX, int NT>
+__global__ void __launch_bounds__(128, 8) batched_octet_kernel(In in, Out out, Mats M, Params P0,
+                                                               const mpf3d_instance *__restrict__ inst, int n_inst,
+                                                               Queue Q, int parity, int32_t *__restrict__ err) {
+    const OctetLane O;
+    for_octets(Q, P0.cells32, parity, [&](uint32_t c, bool active) {
         const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
-        const Params P = instance_params(P0, I);
-        const uint32_t r0 = c - I.offset;
-        const uint32_t plane = (uint32_t)I.nx * (uint32_t)I.ny;
-        const int k = (int)(r0 / plane);
-        const uint32_t r = r0 - (uint32_t)k * plane;
-        const int m = (int)(r / (uint32_t)I.nx);
-        const int l = (int)(r - (uint32_t)m * (uint32_t)I.nx);
-        process_cell<S, AMAX, HEAVY, NT>(in, out, M, P, err, l, m, k);
+        const Place at(c - I.offset, I.nx, I.ny);
+        octet_cell<S, AMAX, NT>(in, out, M, instance_params(P0, I), err, O, active, at.l, at.m, at.k);
+    });
+}
+
+template <int NT>
+__global__ void __launch_bounds__(128, 5) batched_pair_kernel(In in, Out out, Mats M, Params P0,
+                                                              const mpf3d_instance *__restrict__ inst, int n_inst,
+                                                              Queue Q, int parity) {
+    const uint32_t n = *(volatile uint32_t *)(Q.count + 2 * parity + 1);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t c = Q.items[P0.cells32 - 1u - i];
+        const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
+        const Place at(c - I.offset, I.nx, I.ny);
+        pair_cell<NT>(in, out, M, instance_params(P0, I), at.l, at.m, at.k);
     }
+}
+
+// list 2: multi-solid interface cells
+template <int S, int NT>
+__global__ void __launch_bounds__(128, 4) batched_trio_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity) {
+    const uint32_t n = *(volatile uint32_t *)(Q.count + (Q.split ? 4 + parity : 2 * parity + 1));
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        uint32_t &item = Q.items[Q.split ? P0.cells32 + i : P0.cells32 - 1u - i];
+        const uint32_t c = item;
+        const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
+        const Place at(c - I.offset, I.nx, I.ny);
+        if (!trio_cell<S, true, NT>(in, out, M, instance_params(P0, I), at.l, at.m, at.k)) item = c | LEFT;
+    }
+}
+
+// list 0: grain boundaries and junctions, beside the above
+template <int S>
+__global__ void __launch_bounds__(256, 3) batched_general_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity) {
+    const uint32_t n = *(volatile uint32_t *)(Q.count + 2 * parity);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t c = Q.items[i];
+        const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
+        const Place at(c - I.offset, I.nx, I.ny);
+        if (!trio_cell<S, false, 4>(in, out, M, instance_params(P0, I), at.l, at.m, at.k)) Q.items[i] = c | LEFT;
+    }
+}
+
+// what the two left
+template <int S, int AMAX, int NT>
+__global__ void __launch_bounds__(128, 8)
+    batched_rest_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity, int32_t *__restrict__ err) {
+    const OctetLane O;
+    Lists L(Q, parity);
+    if (Q.split) L.n[1] = 0;
+    for_items<8, 32>(
+        L.n[0] + L.n[1] + L.n[2], [&](uint32_t i) { return Q.items[L.item(i, P0.cells32)]; },
+        [](uint32_t c) { return (c & LEFT) == 0u; },
+        [&](uint32_t marked, bool active) {
+            const uint32_t c = marked & ~LEFT;
+            const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
+            const Place at(c - I.offset, I.nx, I.ny);
+            octet_cell<S, AMAX, NT>(in, out, M, instance_params(P0, I), err, O, active, at.l, at.m, at.k);
+        });
+}
+
+// list 0 of the isotropic model, which has no other: what trio_cell leaves is
+// done by the same block
+template <int S, int AMAX>
+__global__ void __launch_bounds__(256, 3)
+    batched_isotropic_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity, int32_t *__restrict__ err) {
+    const OctetLane O;
+    for_items<32, 256>(
+        *(volatile uint32_t *)(Q.count + 2 * parity), [&](uint32_t i) { return Q.items[i]; },
+        [&](uint32_t c) {
+            const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
+            const Place at(c - I.offset, I.nx, I.ny);
+            return trio_cell<S, false, 4>(in, out, M, instance_params(P0, I), at.l, at.m, at.k);
+        },
+        [&](uint32_t c, bool active) {
+            const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
+            const Place at(c - I.offset, I.nx, I.ny);
+            octet_cell<S, AMAX, 4>(in, out, M, instance_params(P0, I), err, O, active, at.l, at.m, at.k);
+        });
 }
 
 // Initial bicrystal: a solid base of height base_height (tanh profile
@@ -1451,10 +1949,9 @@ dim3 zfast_grid(int nx, int ny, int nz, dim3 b) {
 }
 
 
-// A second stream of one device, on which the interface kernel runs beside
-// the general kernel.  The two read only what the sweep wrote and write
-// disjoint cells; both are latency-bound, so running them side by side
-// fills each other's idle issue slots.  Created on first use outside a
+// A second stream of one device, on which pair_kernel runs beside trio_kernel
+// and general_kernel.  They read only what the sweep wrote and write disjoint
+// cells, and fill each other's idle issue slots.  Created on first use outside a
 // stream capture; the fork/join is enqueued under the mutex so that callers
 // on other host threads cannot interleave their event records with it.
 // The second stream of a step and its fork/join events, one set per
@@ -1489,15 +1986,18 @@ bool side_ready(SideStream &side, cudaStream_t s) {
     return side.ready;
 }
 
-// general(stream) and interface(stream) launch the two work-list kernels of
-// a step; with `both`, the interface kernel goes to the caller stream's side stream,
-// forked from s after the sweep and joined back before s continues.
+// Cells from which a step's lists go to pair_kernel, trio_kernel and
+// general_kernel, and what they leave to rest_kernel; on smaller domains the
+// octets take everything.  us per step by octets / by kind, with one grain per
+// 1000 surface cells: 64 x 64 x 64 31 / 46, 96 x 96 x 64 47 / 49, 128^3 89 / 59;
+// 150 x 117 x 90 isotropic 86 / 31.
+constexpr int64_t PAIR_CELLS = 1 << 19;
+
+// general(stream) and interface(stream) launch the work-list kernels of a step;
+// interface's go to the caller stream's side stream, forked from s after the
+// sweep and joined back before s continues.
 template <class General, class Interface>
-void launch_side_by_side(cudaStream_t s, bool both, General &&general, Interface &&interface) {
-    if (!both) {
-        general(s);
-        return;
-    }
+void launch_side_by_side(cudaStream_t s, General &&general, Interface &&interface) {
     int dev = 0;
     cudaGetDevice(&dev);
     SideTable &tab = side_table_of(dev);
@@ -1568,18 +2068,30 @@ void launch_step(const In &in, const Out &out, const Mats &M, const Params &P, c
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const dim3 g_general(sms * T.general_blocks_per_sm), g_iface(sms * T.iface_blocks_per_sm);
+    if (P.cells < PAIR_CELLS) {  // 8 blocks of 128 threads are resident per SM
+        if (P.sym_normals) octet_kernel<S, AMAX, 4><<<sms * 8, 128, 0, s>>>(in, out, M, P, Q, parity, err);
+        else octet_kernel<S, AMAX, 8><<<sms * 8, 128, 0, s>>>(in, out, M, P, Q, parity, err);
+        return;
+    }
+    const int g_general = sms * T.general_blocks_per_sm, g_iface = sms * T.iface_blocks_per_sm;
+    if (!P.use_aniso) {
+        isotropic_kernel<S, AMAX><<<g_general, T.general_threads, 0, s>>>(in, out, M, P, Q, parity, err);
+        return;
+    }
     launch_side_by_side(
-        s, P.use_aniso,
+        s,
         [&](cudaStream_t st) {
-            general_kernel<S, AMAX><<<g_general, T.general_threads, 0, st>>>(in, out, M, P, Q, parity, err);
+            if (P.sym_normals) trio_kernel<S, 4><<<g_iface, T.iface_threads, 0, st>>>(in, out, M, P, Q, parity);
+            else trio_kernel<S, 8><<<g_iface, T.iface_threads, 0, st>>>(in, out, M, P, Q, parity);
+            general_kernel<S><<<g_general, T.general_threads, 0, st>>>(in, out, M, P, Q, parity);
         },
         [&](cudaStream_t st) {
-            if (P.sym_normals)
-                interface_kernel<S, AMAX, 4><<<g_iface, T.iface_threads, 0, st>>>(in, out, M, P, Q, parity, err);
-            else
-                interface_kernel<S, AMAX, 8><<<g_iface, T.iface_threads, 0, st>>>(in, out, M, P, Q, parity, err);
+            if (!Q.split) return;
+            if (P.sym_normals) pair_kernel<4><<<g_iface, T.iface_threads, 0, st>>>(in, out, M, P, Q, parity);
+            else pair_kernel<8><<<g_iface, T.iface_threads, 0, st>>>(in, out, M, P, Q, parity);
         });
+    if (P.sym_normals) rest_kernel<S, AMAX, 4><<<sms * 8, 128, 0, s>>>(in, out, M, P, Q, parity, err);
+    else rest_kernel<S, AMAX, 8><<<sms * 8, 128, 0, s>>>(in, out, M, P, Q, parity, err);
 }
 
 bool tuning_ok(const mpf3d_tuning &T) {
@@ -1590,7 +2102,12 @@ bool tuning_ok(const mpf3d_tuning &T) {
            (T.iface_threads == 64 || T.iface_threads == 128);
 }
 
-const mpf3d_tuning kDefaultTuning = {4, 8, 8, 256, 8, 128};
+// Launch shape of a step (single or batched) without mpf3d_tuning: blocks of 128 threads, all of
+// them resident in one or two waves.  (us per step at 256^3 / 512 x 512 x 256 /
+// 128^3 with general and interface grids of 16 x 128 threads per SM: 147 / 343 /
+// 57; with 8 x 256 and 64 x 64: 153 / 347 / 60; with 8 x 256 and 8 x 128: 148 /
+// 349 / 58.)
+constexpr mpf3d_tuning DEFAULT_TUNING = {4, 8, 16, 128, 16, 128};
 
 }  // namespace
 
@@ -1722,18 +2239,30 @@ void launch_batched(const In &in, const Out &out, const Mats &M, const Params &P
     // gain here; the work-list grids come from T (the sweep's 32 x 8 x 4
     // tiles are fixed by the instance table)
     const int sms = sms_of_current_device();
-    batched_queue_kernel<S, AMAX, false><<<sms * T.general_blocks_per_sm, T.general_threads, 0, s>>>(
-        in, out, M, P0, inst, n_inst, Q, parity, err);
-    if (P0.use_aniso && P0.sym_normals)
-        batched_queue_kernel<S, AMAX, true, 4><<<sms * T.iface_blocks_per_sm, T.iface_threads, 0, s>>>(
-            in, out, M, P0, inst, n_inst, Q, parity, err);
-    else if (P0.use_aniso)
-        batched_queue_kernel<S, AMAX, true, 8><<<sms * T.iface_blocks_per_sm, T.iface_threads, 0, s>>>(
-            in, out, M, P0, inst, n_inst, Q, parity, err);
+    const int g_iface = sms * T.iface_blocks_per_sm, g_general = sms * T.general_blocks_per_sm;
+    if (P0.cells < PAIR_CELLS) {  // as the single domain's step
+        if (P0.sym_normals)
+            batched_octet_kernel<S, AMAX, 4><<<sms * 8, 128, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity, err);
+        else batched_octet_kernel<S, AMAX, 8><<<sms * 8, 128, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity, err);
+        return;
+    }
+    if (!P0.use_aniso) {
+        batched_isotropic_kernel<S, AMAX>
+            <<<g_general, T.general_threads, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity, err);
+        return;
+    }
+#define BATCHED(NT)                                                                                                   \
+    do {                                                                                                              \
+        if (Q.split)                                                                                                  \
+            batched_pair_kernel<NT><<<g_iface, T.iface_threads, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity);     \
+        batched_trio_kernel<S, NT><<<g_iface, T.iface_threads, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity);      \
+        batched_general_kernel<S><<<g_general, T.general_threads, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity);   \
+        batched_rest_kernel<S, AMAX, NT><<<sms * 8, 128, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity, err);       \
+    } while (0)
+    if (P0.sym_normals) BATCHED(4);
+    else BATCHED(8);
+#undef BATCHED
 }
-
-// launch shape of the batched step before it was tuned
-const mpf3d_tuning kBatchedDefault = {4, 8, 8, 256, 8, 128};
 
 }  // namespace
 
@@ -1755,7 +2284,7 @@ static int compact_step_impl(const uint32_t *cnt, const uint16_t *idx, const flo
                              uint32_t *work_count, int parity, int32_t *err, void *stream,
                              const mpf3d_tuning *tuning, uint8_t *tile_flags, int options, mpf3d_step_clock *clock,
                              double clock_T_melt, double clock_rate) {
-    const mpf3d_tuning T = tuning ? *tuning : kDefaultTuning;
+    const mpf3d_tuning T = tuning ? *tuning : DEFAULT_TUNING;
     if (!tuning_ok(T)) return MPF3D_ERR_ARG;
     if (!cnt || !idx || !val || !cnt_out || !idx_out || !val_out || !T0z || !wij || !a2ij || !mij || !n111 || !sc ||
         !err || !work_items || !work_count)
@@ -1878,7 +2407,7 @@ extern "C" int mpf3d_batched_step_tuned(const uint32_t *head, const uint16_t *id
                                         int symmetric_normals, uint32_t *work_items, uint32_t *work_count, int parity,
                                         int32_t *err, void *stream, int options, const mpf3d_tuning *tuning,
                                         uint8_t *tile_flags) {
-    const mpf3d_tuning T = tuning ? *tuning : kBatchedDefault;
+    const mpf3d_tuning T = tuning ? *tuning : DEFAULT_TUNING;
     if (!tuning_ok(T)) return MPF3D_ERR_ARG;
     if (!head || !idx || !val || !head_out || !idx_out || !val_out || !inst || !wij || !a2ij || !mij || !n111 ||
         !sc || !err || !work_items || !work_count || n_inst <= 0 || n_tiles <= 0 || total_cells == 0 || N <= 0 ||

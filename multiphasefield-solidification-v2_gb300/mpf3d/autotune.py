@@ -19,7 +19,7 @@ import os
 
 from . import _lib
 
-DEFAULT = (4, 8, 8, 256, 8, 128)
+DEFAULT = (4, 8, 16, 128, 16, 128)
 SWEEP = [(zb, by) for zb in (2, 4, 8) for by in (4, 8, 16)]
 QUEUE = [(g, gt, i, it) for (g, gt), (i, it) in itertools.product([(4, 256), (8, 256), (16, 128), (32, 128)],
                                                                    [(4, 128), (8, 128), (16, 64), (32, 64)])]
