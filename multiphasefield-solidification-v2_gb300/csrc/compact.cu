@@ -941,10 +941,11 @@ __device__ __forceinline__ void octet_cell(const In &in, const Out &out, const M
 // to the front -- so that the general update runs with converged warps.
 constexpr int SWEEP_ZB = 4;  // cells per thread along z (default; batches always use it)
 
-// Where the sweep sends a queued cell: list 0 (general), 1 (interface) or 2
-// (interface with several solids).  BlockSink counts a block's cells per
-// list in shared memory (one shared atomic per warp, cell and list) and
-// keeps each cell's list and offset in registers; the block then reserves
+// Where the sweep sends its cells: 0 for one it wrote itself, else 1 + the
+// list (0 general, 1 interface, 2 interface with several solids), two bits per
+// cell of a thread's column.  BlockSink counts a block's cells per list in
+// shared memory (one shared atomic per warp and list, over the warp's whole
+// column) and keeps each cell's offset in registers; the block then reserves
 // its segments with one global atomic per list and writes the cell indices
 // (flush).  The counters are one address each, and per-warp global atomics
 // from every SM queued up at the L2 slice that holds them.  Cells are
@@ -954,29 +955,31 @@ template <int ZB>
 struct BlockSink {
     uint32_t *cnt;     // shared: cells of the block per list
     uint32_t off[ZB];  // cell j's position in its list's block segment
-    int lst[ZB];       // cell j's list, -1 if it is not queued
+    uint32_t codes;
 
-    __device__ __forceinline__ explicit BlockSink(uint32_t *c) : cnt(c) {
+    __device__ __forceinline__ explicit BlockSink(uint32_t *c) : cnt(c), codes(0) {}
+    // by all lanes of a warp
+    __device__ __forceinline__ void add(uint32_t column) {
+        codes = column;
+        if (!__any_sync(0xffffffffu, column)) return;
+        const unsigned before = (1u << (threadIdx.x & 31)) - 1u;
 #pragma unroll
-        for (int j = 0; j < ZB; ++j) {
-            off[j] = 0;
-            lst[j] = -1;
-        }
-    }
-    __device__ __forceinline__ void add(int j, int list, uint32_t) {
-        const unsigned am = __activemask();
-        const int lane = threadIdx.x & 31;
+        for (uint32_t L = 1; L <= 3; ++L) {
+            uint32_t total = 0, at[ZB];
 #pragma unroll
-        for (int L = 0; L < 3; ++L) {
-            const unsigned bm = __ballot_sync(am, list == L);
-            if (!bm) continue;
-            const int leader = __ffs(bm) - 1;
+            for (int j = 0; j < ZB; ++j) {
+                const unsigned bm = __ballot_sync(0xffffffffu, (column >> (2 * j) & 3u) == L);
+                at[j] = total + __popc(bm & before);
+                total += __popc(bm);
+            }
+            if (!total) continue;
             uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(cnt + L, (uint32_t)__popc(bm));
-            base = __shfl_sync(am, base, leader);
-            if (list == L) off[j] = base + (uint32_t)__popc(bm & ((1u << lane) - 1u));
+            if ((threadIdx.x & 31) == 0) base = atomicAdd(cnt + L - 1, total);
+            base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll
+            for (int j = 0; j < ZB; ++j)
+                if ((column >> (2 * j) & 3u) == L) off[j] = base + at[j];
         }
-        lst[j] = list;
     }
     // after the block's adds and a barrier: base[L] is the block's first
     // position in list L; cell j is (k0 + j) * plane + col
@@ -984,79 +987,60 @@ struct BlockSink {
                                           uint32_t col, int k0) const {
 #pragma unroll
         for (int j = 0; j < ZB; ++j) {
-            if (lst[j] < 0) continue;
-            const uint32_t pos = base[lst[j]] + off[j];
+            const uint32_t code = codes >> (2 * j) & 3u;
+            if (!code) continue;
+            const uint32_t pos = base[code - 1] + off[j];
             const uint32_t c = (uint32_t)(k0 + j) * plane + col;
-            Q.items[lst[j] == 0 ? pos : (lst[j] == 1 ? cells - 1u - pos : cells + pos)] = c;
+            Q.items[code == 1 ? pos : (code == 2 ? cells - 1u - pos : cells + pos)] = c;
         }
     }
 };
 
-// Classification of cell c = (l, m, k0 + j) from its head h0 and its 6
-// neighbours' heads hn = {x+, x-, y+, y-, z+, z-} (z clamped: a neighbour
-// beyond the domain is the cell itself): a uniform neighbourhood is written
-// directly; any other cell goes to a work list.  Returns whether uniform.
-template <class Sink>
-__device__ __forceinline__ bool sweep_cell(const In &in, const Out &out, const Params &P, bool split, Sink &sink,
-                                           int j, uint32_t c, uint32_t h0, const uint32_t (&hn)[6],
-                                           const uint32_t (&qn)[6]) {
-    bool uniform = hcount(h0) == 1 && !hexplicit(h0);
+// Classification of a cell c from its head h0 and its 6 neighbours' heads hn =
+// {x+, x-, y+, y-, z+, z-} at qn (z clamped: a neighbour beyond the domain is the
+// cell itself): a uniform neighbourhood is written directly, any other cell goes
+// to a work list.  Returns the cell's code.
+__device__ __forceinline__ uint32_t sweep_cell(const In &in, const Out &out, const Params &P, bool split, uint32_t c,
+                                               uint32_t h0, const uint32_t (&hn)[6], const uint32_t (&qn)[6]) {
+    const uint32_t h[7] = {h0, hn[0], hn[1], hn[2], hn[3], hn[4], hn[5]};
+    uint32_t differ = 0, any = 0, least = 0xffffffffu;
 #pragma unroll
-    for (int p = 0; p < 6; ++p) uniform = uniform && hn[p] == h0;
-    if (uniform) {
+    for (int p = 0; p < 7; ++p) {
+        differ |= h[p] ^ h0;
+        any |= h[p];
+        least = min(least, h[p] - 1u);
+    }
+    if (differ == 0 && (h0 & 0xffu) == 1u) {
         // the one phase of the neighbourhood keeps the cell at exactly 1
         out.head[c] = h0;
-        return true;
+        return 0;
     }
-    bool liq = hcount(h0) > 0 && hid0(h0) == LIQ;
-    bool sol = hcount(h0) > 1 || (hcount(h0) == 1 && hid0(h0) != LIQ);
+    // Liquid somewhere: a head with phases and first id 0 is 1..255 (an empty one
+    // is 0).  A solid somewhere: a first id beyond 0, or a count beyond 1.
+    const bool heavy = P.use_aniso && least < 0xffu && (any & ~0x81u) != 0u;
+    if (!heavy) return 1;
+    if (!split) return 2;
+    // Several solids: more than one in a cell (3 phases, or 2 without liquid), or
+    // different ones in two; the solid beside the liquid of a two-phase cell is
+    // its second id (head 2: first id 0, count 2).
+    uint32_t second[7], most = 0, hi = 0, lo = 0xffffffffu;
 #pragma unroll
-    for (int p = 0; p < 6; ++p) {
-        const uint32_t h = hn[p];
-        liq = liq || (hcount(h) > 0 && hid0(h) == LIQ);
-        sol = sol || hcount(h) > 1 || (hcount(h) == 1 && hid0(h) != LIQ);
+    for (int p = 0; p < 7; ++p)
+        second[p] = h[p] == 2u ? (uint32_t)__ldg(in.idx + P.cells32 + (p == 0 ? c : qn[p == 0 ? 0 : p - 1])) : h[p] >> 8;
+#pragma unroll
+    for (int p = 0; p < 7; ++p) {
+        most = max(most, (h[p] & 0x7fu) + (h[p] >> 8 ? 1u : 0u));
+        hi = max(hi, second[p]);
+        lo = min(lo, second[p] - 1u);
     }
-    const bool heavy = liq && sol && P.use_aniso;
-    bool multi = false;
-    if (heavy && split) {
-        // several solids in the active list: a head with 3+ phases or two
-        // solids, two different solid first ids, or -- read only where the
-        // heads do not tell -- different solids beside the liquid
-        int sid = -1;
-        const uint32_t hs[7] = {h0, hn[0], hn[1], hn[2], hn[3], hn[4], hn[5]};
-        const uint32_t qs[7] = {c, qn[0], qn[1], qn[2], qn[3], qn[4], qn[5]};
-#pragma unroll
-        for (int p = 0; p < 7; ++p) {
-            const int cn = hcount(hs[p]), id = hid0(hs[p]);
-            if (cn >= 3 || (cn == 2 && id != LIQ)) multi = true;
-            else if (cn >= 1 && id != LIQ) {
-                if (sid < 0) sid = id;
-                else if (sid != id) multi = true;
-            }
-        }
-        if (!multi) {
-            int second[7];
-#pragma unroll
-            for (int p = 0; p < 7; ++p)
-                second[p] = hcount(hs[p]) == 2 ? (int)__ldg(in.idx + P.cells32 + qs[p]) : -1;
-#pragma unroll
-            for (int p = 0; p < 7; ++p) {
-                if (second[p] < 0) continue;
-                if (sid < 0) sid = second[p];
-                else if (sid != second[p]) multi = true;
-            }
-        }
-    }
-    sink.add(j, heavy ? (multi ? 2 : 1) : 0, c);
-    return false;
+    return most > 2u || hi != lo + 1u ? 3 : 2;
 }
 
 // The sweep of one column of ZB cells (l, m, k0..k0+ZB-1) of a domain;
-// returns whether every one of them was uniform (cells past the top count
-// as uniform).
-template <int ZB = SWEEP_ZB, class Sink>
-__device__ __forceinline__ bool sweep_column(const In &in, const Out &out, const Params &P, bool split, Sink &sink,
-                                             int l, int m, int k0) {
+// returns their codes (cells past the top count as written).
+template <int ZB = SWEEP_ZB>
+__device__ __forceinline__ uint32_t sweep_column(const In &in, const Out &out, const Params &P, bool split, int l,
+                                                 int m, int k0) {
     const uint32_t plane = (uint32_t)P.nx * (uint32_t)P.ny;
     const uint32_t col = P.base + (uint32_t)m * (uint32_t)P.nx + (uint32_t)l;
     const uint32_t dxp = (l < P.nx - 1) ? 1u : (uint32_t)(1 - P.nx);
@@ -1065,7 +1049,7 @@ __device__ __forceinline__ bool sweep_column(const In &in, const Out &out, const
     const uint32_t dym = (m > 0) ? (uint32_t)(-P.nx) : (uint32_t)((P.ny - 1) * P.nx);
     // heads of the column k0-1 .. k0+ZB (z clamped)
     uint32_t hz[ZB + 2];
-    bool all_uniform = true;
+    uint32_t codes = 0;
 #pragma unroll
     for (int j = 0; j < ZB + 2; ++j) {
         const int kk = min(max(k0 - 1 + j, 0), P.nz - 1);
@@ -1086,9 +1070,9 @@ __device__ __forceinline__ bool sweep_column(const In &in, const Out &out, const
         if (k == P.nz - 1) hn[4] = h0;
         if (k == 0) hn[5] = h0;
         const uint32_t qn[6] = {qxp, qxm, qyp, qym, k < P.nz - 1 ? c + plane : c, k > 0 ? c - plane : c};
-        all_uniform = sweep_cell(in, out, P, split, sink, j, c, h0, hn, qn) && all_uniform;
+        codes |= sweep_cell(in, out, P, split, c, h0, hn, qn) << (2 * j);
     }
-    return all_uniform;
+    return codes;
 }
 
 // The same sweep reading the heads from a shared-memory tile: the block's
@@ -1097,15 +1081,15 @@ __device__ __forceinline__ bool sweep_column(const In &in, const Out &out, const
 // layers from k0 - 1; the periodic x and y halos patched in after the copy).
 constexpr int TMA_X = 40;
 
-template <int ZB, class Sink>
-__device__ __forceinline__ bool sweep_column_tile(const uint32_t *tile, int rows, const In &in, const Out &out,
-                                                  const Params &P, bool split, Sink &sink, int l, int m, int k0,
-                                                  int l0, int m0) {
+template <int ZB>
+__device__ __forceinline__ uint32_t sweep_column_tile(const uint32_t *tile, int rows, const In &in, const Out &out,
+                                                      const Params &P, bool split, int l, int m, int k0, int l0,
+                                                      int m0) {
     const uint32_t plane = (uint32_t)P.nx * (uint32_t)P.ny;
     const uint32_t col = (uint32_t)m * (uint32_t)P.nx + (uint32_t)l;
     const int xi = l - l0 + 4, yi = m - m0 + 1;
     auto at = [&](int x, int y, int z) { return tile[(z * rows + y) * TMA_X + x]; };
-    bool all_uniform = true;
+    uint32_t codes = 0;
 #pragma unroll
     for (int j = 0; j < ZB; ++j) {
         const int k = k0 + j;
@@ -1123,9 +1107,9 @@ __device__ __forceinline__ bool sweep_column_tile(const uint32_t *tile, int rows
                                 row + (uint32_t)wrap_p(m, P.ny) * (uint32_t)P.nx + (uint32_t)l,
                                 row + (uint32_t)wrap_m(m, P.ny) * (uint32_t)P.nx + (uint32_t)l,
                                 k < P.nz - 1 ? c + plane : c, k > 0 ? c - plane : c};
-        all_uniform = sweep_cell(in, out, P, split, sink, j, c, h0, hn, qn) && all_uniform;
+        codes |= sweep_cell(in, out, P, split, c, h0, hn, qn) << (2 * j);
     }
-    return all_uniform;
+    return codes;
 }
 
 // Quiet tiles.  A tile is the 32 x 1 x ZB cells one warp of the sweep
@@ -1182,7 +1166,7 @@ __global__ void __launch_bounds__(512, 3) sweep_kernel(In in, Out out, Mats M, P
     // branch below is warp-uniform except l < nx
     if (m < P.ny && k0 < P.nz) {
         if (!T.flags) {
-            if (l < P.nx) sweep_column<ZB>(in, out, P, Q.split, sink, l, m, k0);
+            sink.add(l < P.nx ? sweep_column<ZB>(in, out, P, Q.split, l, m, k0) : 0u);
         } else {
             const int tx = (int)blockIdx.x, kb = k0 / ZB;
             const uint8_t *fin = T.flags + (size_t)(parity ^ 1) * T.n;
@@ -1204,8 +1188,8 @@ __global__ void __launch_bounds__(512, 3) sweep_kernel(In in, Out out, Mats M, P
             if (quiet) {
                 if (lane0) fout[t] = 1;
             } else {
-                const bool uni = l < P.nx ? sweep_column<ZB>(in, out, P, Q.split, sink, l, m, k0) : true;
-                const bool all = __all_sync(0xffffffffu, uni);
+                sink.add(l < P.nx ? sweep_column<ZB>(in, out, P, Q.split, l, m, k0) : 0u);
+                const bool all = __all_sync(0xffffffffu, sink.codes == 0u);
                 if (lane0) fout[t] = all ? 1 : 0;
             }
         }
@@ -1356,13 +1340,12 @@ __global__ void __launch_bounds__(512, 3) sweep_kernel_tma(const __grid_constant
     BlockSink<ZB> sink(s_cnt);
     if (row_ok && staged) {
         if (!T.flags) {
-            if (l < P.nx) sweep_column_tile<ZB>(tile, rows, in, out, P, Q.split, sink, l, m, k0, l0, m0);
+            sink.add(l < P.nx ? sweep_column_tile<ZB>(tile, rows, in, out, P, Q.split, l, m, k0, l0, m0) : 0u);
         } else if (quiet) {
             if (threadIdx.x == 0) fout[t] = 1;
         } else {
-            const bool uni = l < P.nx ? sweep_column_tile<ZB>(tile, rows, in, out, P, Q.split, sink, l, m, k0, l0, m0)
-                                      : true;
-            const bool all = __all_sync(0xffffffffu, uni);
+            sink.add(l < P.nx ? sweep_column_tile<ZB>(tile, rows, in, out, P, Q.split, l, m, k0, l0, m0) : 0u);
+            const bool all = __all_sync(0xffffffffu, sink.codes == 0u);
             if (threadIdx.x == 0) fout[t] = all ? 1 : 0;
         }
     } else if (row_ok && quiet && threadIdx.x == 0) {
@@ -1674,7 +1657,7 @@ __global__ void __launch_bounds__(256) batched_sweep_kernel(In in, Out out, Para
     const Params P = instance_params(P0, I);
     BlockSink<SWEEP_ZB> sink(s_cnt);
     if (!flags) {
-        if (inside) sweep_column(in, out, P, Q.split, sink, l, m, k0);
+        if (row_in) sink.add(inside ? sweep_column(in, out, P, Q.split, l, m, k0) : 0u);
     } else {
         const uint32_t nw = gridDim.x * 8u;
         const uint8_t *fin = flags + (size_t)(parity ^ 1) * nw;
@@ -1699,8 +1682,8 @@ __global__ void __launch_bounds__(256) batched_sweep_kernel(In in, Out out, Para
             if ((f0 & f1 & f2 & f3 & f4 & f5 & f6) != 0u) {
                 if (lane0) fout[w] = 1;
             } else {
-                const bool uni = l < I.nx ? sweep_column(in, out, P, Q.split, sink, l, m, k0) : true;
-                const bool all = __all_sync(0xffffffffu, uni);
+                sink.add(inside ? sweep_column(in, out, P, Q.split, l, m, k0) : 0u);
+                const bool all = __all_sync(0xffffffffu, sink.codes == 0u);
                 if (lane0) fout[w] = all ? 1 : 0;
             }
         }
