@@ -956,11 +956,14 @@ struct BlockSink {
     uint32_t *cnt;     // shared: cells of the block per list
     uint32_t off[ZB];  // cell j's position in its list's block segment
     uint32_t codes;
+    uint32_t cell, plane;  // cell j is cell + j * plane
 
     __device__ __forceinline__ explicit BlockSink(uint32_t *c) : cnt(c), codes(0) {}
     // by all lanes of a warp
-    __device__ __forceinline__ void add(uint32_t column) {
+    __device__ __forceinline__ void add(uint32_t column, uint32_t cell0, uint32_t stride) {
         codes = column;
+        cell = cell0;
+        plane = stride;
         if (!__any_sync(0xffffffffu, column)) return;
         const unsigned before = (1u << (threadIdx.x & 31)) - 1u;
 #pragma unroll
@@ -982,15 +985,14 @@ struct BlockSink {
         }
     }
     // after the block's adds and a barrier: base[L] is the block's first
-    // position in list L; cell j is (k0 + j) * plane + col
-    __device__ __forceinline__ void flush(const Queue &Q, uint32_t cells, const uint32_t *base, uint32_t plane,
-                                          uint32_t col, int k0) const {
+    // position in list L
+    __device__ __forceinline__ void flush(const Queue &Q, uint32_t cells, const uint32_t *base) const {
 #pragma unroll
         for (int j = 0; j < ZB; ++j) {
             const uint32_t code = codes >> (2 * j) & 3u;
             if (!code) continue;
             const uint32_t pos = base[code - 1] + off[j];
-            const uint32_t c = (uint32_t)(k0 + j) * plane + col;
+            const uint32_t c = cell + (uint32_t)j * plane;
             Q.items[code == 1 ? pos : (code == 2 ? cells - 1u - pos : cells + pos)] = c;
         }
     }
@@ -1142,68 +1144,113 @@ __device__ __forceinline__ void advance_clock(const Params &P) {
     P.clock->step[P.parity ^ 1] = s + 1;
 }
 
-// 40 registers (3 blocks of 512 per SM): more resident warps beat keeping
-// ZB = 8 columns in registers; the tuner then prefers ZB = 4
-template <int S, int AMAX, int ZB = SWEEP_ZB>
-__global__ void __launch_bounds__(512, 3) sweep_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity,
-                                                    Tiles T, int32_t *__restrict__ err) {
-    __shared__ uint32_t s_cnt[3], s_base[3];
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    const int m = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k0 = (blockIdx.z * blockDim.z + threadIdx.z) * ZB;
-    const int tlin = threadIdx.x + (int)blockDim.x * threadIdx.y;  // blockDim.z is 1
+// The sweep's tiles in chunks of blockDim.y rows; a block takes every
+// gridDim.x-th chunk, at most SWEEP_TILES tiles (distant ones: the tiles that are
+// not quiet lie together).  A lane per tile reads its flags (quiet), then the warps
+// share the others, one per warp and round; visit fills the warp's sink, flag_of
+// is a tile's place in fout.  A warp of its own for each of the 79 % quiet tiles of
+// a 256^3 step with 64 grains spent the time on starting blocks; us per step with a
+// block per chunk / with up to 128 tiles per block: 256^3 41 / 23, 512 x 512 x 256
+// 155 / 63 (64 tiles: 69, 32: 78), 24 bicrystals 92 / 79.  With consecutive chunks
+// per block, 256^3 took 43: blocks whose tiles are all visited came last.
+constexpr uint32_t SWEEP_TILES = 128;  // blocks have at least as many threads
+
+template <int ZB, class Flag, class Quiet, class Visit>
+__device__ __forceinline__ void sweep_tiles(const Queue &Q, uint32_t cells, int parity, uint32_t chunks,
+                                            uint8_t *__restrict__ fout, Flag &&flag_of, Quiet &&quiet, Visit &&visit) {
+    __shared__ uint32_t s_cnt[3], s_base[3], s_tile[SWEEP_TILES], s_n;
+    const uint32_t lane = threadIdx.x, tlin = lane + 32u * threadIdx.y, rows = blockDim.y;
     if (tlin < 3) s_cnt[tlin] = 0;
-    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && tlin == 3 && threadIdx.z == 0) advance_clock(P);
-    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x < 2 && threadIdx.y == 0 &&
-        threadIdx.z == 0)
-        Q.count[2 * (parity ^ 1) + threadIdx.x] = 0;  // the previous step's kernels are done with them
-    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 2 && threadIdx.y == 0 &&
-        threadIdx.z == 0 && Q.split)
-        Q.count[4 + (parity ^ 1)] = 0;
+    if (tlin == 3) s_n = 0;
     __syncthreads();
-    BlockSink<ZB> sink(s_cnt);
-    // a warp is one threadIdx.y row: its 32 lanes share m and k0, so every
-    // branch below is warp-uniform except l < nx
-    if (m < P.ny && k0 < P.nz) {
-        if (!T.flags) {
-            sink.add(l < P.nx ? sweep_column<ZB>(in, out, P, Q.split, l, m, k0) : 0u);
-        } else {
-            const int tx = (int)blockIdx.x, kb = k0 / ZB;
-            const uint8_t *fin = T.flags + (size_t)(parity ^ 1) * T.n;
-            uint8_t *fout = T.flags + (size_t)parity * T.n;
-            auto tid = [&](int a, int b, int c) {
-                return ((uint32_t)c * (uint32_t)P.ny + (uint32_t)b) * (uint32_t)T.ntx + a;
-            };
-            const uint32_t t = tid(tx, m, kb);
-            // the 7 flags are loaded together (no short-circuit chain of loads)
-            const uint32_t f0 = fin[t];
-            const uint32_t f1 = fin[tid(tx + 1 < T.ntx ? tx + 1 : 0, m, kb)];
-            const uint32_t f2 = fin[tid(tx > 0 ? tx - 1 : T.ntx - 1, m, kb)];
-            const uint32_t f3 = fin[tid(tx, m + 1 < P.ny ? m + 1 : 0, kb)];
-            const uint32_t f4 = fin[tid(tx, m > 0 ? m - 1 : P.ny - 1, kb)];
-            const uint32_t f5 = fin[tid(tx, m, kb + 1 < T.nkb ? kb + 1 : kb)];
-            const uint32_t f6 = fin[tid(tx, m, kb > 0 ? kb - 1 : kb)];
-            const bool quiet = (f0 & f1 & f2 & f3 & f4 & f5 & f6) != 0u;
-            const bool lane0 = (threadIdx.x & 31) == 0;
-            if (quiet) {
-                if (lane0) fout[t] = 1;
-            } else {
-                sink.add(l < P.nx ? sweep_column<ZB>(in, out, P, Q.split, l, m, k0) : 0u);
+    if (32u * threadIdx.y < SWEEP_TILES) {
+        const uint32_t chunk = blockIdx.x + tlin / rows * gridDim.x, row = tlin % rows;
+        const bool in = chunk < chunks;
+        const bool skip = in && quiet(chunk, row);
+        if (skip && fout) fout[flag_of(chunk, row)] = 1;
+        const unsigned mask = __ballot_sync(0xffffffffu, in && !skip);
+        uint32_t at = 0;
+        if (lane == 0 && mask) at = atomicAdd(&s_n, (uint32_t)__popc(mask));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (mask >> lane & 1u) s_tile[at + __popc(mask & ((1u << lane) - 1u))] = chunk * rows + row;
+    }
+    __syncthreads();
+    const uint32_t n = s_n;
+    for (uint32_t r = 0; r < n; r += rows) {
+        BlockSink<ZB> sink(s_cnt);
+        if (r + threadIdx.y < n) {
+            const uint32_t t = s_tile[r + threadIdx.y], chunk = t / rows, row = t - chunk * rows;
+            visit(chunk, row, sink);
+            if (fout) {
                 const bool all = __all_sync(0xffffffffu, sink.codes == 0u);
-                if (lane0) fout[t] = all ? 1 : 0;
+                if (lane == 0) fout[flag_of(chunk, row)] = all ? 1 : 0;
             }
         }
+        __syncthreads();
+        if (tlin < 3) {
+            const uint32_t k = s_cnt[tlin];
+            uint32_t *ctr = tlin == 2 ? Q.count + 4 + parity : Q.count + 2 * parity + tlin;
+            s_base[tlin] = k ? atomicAdd(ctr, k) : 0u;
+            s_cnt[tlin] = 0;
+        }
+        __syncthreads();
+        sink.flush(Q, cells, s_base);
     }
-    __syncthreads();
-    if (tlin < 3) {
-        const uint32_t n = s_cnt[tlin];
-        uint32_t *ctr = tlin == 2 ? Q.count + 4 + parity : Q.count + 2 * parity + tlin;
-        s_base[tlin] = n ? atomicAdd(ctr, n) : 0u;
+}
+
+// the other parity's counters, which the previous step's kernels are done with
+__device__ __forceinline__ void clear_counters(const Queue &Q, int parity, uint32_t t) {
+    if (t < 2) Q.count[2 * (parity ^ 1) + t] = 0;
+    if (t == 2 && Q.split) Q.count[4 + (parity ^ 1)] = 0;
+}
+
+// 40 registers (3 blocks of 512 per SM): more resident warps beat keeping
+// ZB = 8 columns in registers; the tuner then prefers ZB = 4
+template <int ZB>
+__global__ void __launch_bounds__(512, 3) sweep_kernel(In in, Out out, Params P, Queue Q, int parity, Tiles T,
+                                                       uint32_t chunks) {
+    if (blockIdx.x == 0) {
+        const uint32_t t = threadIdx.x + 32u * threadIdx.y;
+        clear_counters(Q, parity, t);
+        if (t == 3) advance_clock(P);
     }
-    __syncthreads();
-    if (l < P.nx && m < P.ny && k0 < P.nz)
-        sink.flush(Q, P.cells32, s_base, (uint32_t)P.nx * (uint32_t)P.ny,
-                   P.base + (uint32_t)m * (uint32_t)P.nx + (uint32_t)l, k0);
+    const uint8_t *fin = T.flags + (size_t)(parity ^ 1) * T.n;
+    uint8_t *fout = T.flags ? T.flags + (size_t)parity * T.n : nullptr;
+    const uint32_t ntx = (uint32_t)T.ntx, bands = ((uint32_t)P.ny + blockDim.y - 1u) / blockDim.y;
+    struct Tile {
+        int tx, m, kb;
+    };
+    auto tile_of = [&](uint32_t chunk, uint32_t row) {  // chunks: x first, then bands of rows, then z
+        const uint32_t q = chunk / ntx, kb = q / bands;
+        return Tile{(int)(chunk - q * ntx), (int)((q - kb * bands) * blockDim.y + row), (int)kb};
+    };
+    auto at = [&](int a, int b, int c) { return ((uint32_t)c * (uint32_t)P.ny + (uint32_t)b) * ntx + (uint32_t)a; };
+    sweep_tiles<ZB>(
+        Q, P.cells32, parity, chunks, fout,
+        [&](uint32_t chunk, uint32_t row) {
+            const Tile t = tile_of(chunk, row);
+            return at(t.tx, t.m, t.kb);
+        },
+        [&](uint32_t chunk, uint32_t row) {
+            const auto [tx, m, kb] = tile_of(chunk, row);
+            if (!T.flags || m >= P.ny) return false;
+            // the 7 flags are loaded together (no short-circuit chain of loads)
+            const uint32_t f0 = fin[at(tx, m, kb)];
+            const uint32_t f1 = fin[at(tx + 1 < T.ntx ? tx + 1 : 0, m, kb)];
+            const uint32_t f2 = fin[at(tx > 0 ? tx - 1 : T.ntx - 1, m, kb)];
+            const uint32_t f3 = fin[at(tx, m + 1 < P.ny ? m + 1 : 0, kb)];
+            const uint32_t f4 = fin[at(tx, m > 0 ? m - 1 : P.ny - 1, kb)];
+            const uint32_t f5 = fin[at(tx, m, kb + 1 < T.nkb ? kb + 1 : kb)];
+            const uint32_t f6 = fin[at(tx, m, kb > 0 ? kb - 1 : kb)];
+            return (f0 & f1 & f2 & f3 & f4 & f5 & f6) != 0u;
+        },
+        [&](uint32_t chunk, uint32_t row, BlockSink<ZB> &sink) {
+            const Tile t = tile_of(chunk, row);
+            const uint32_t plane = (uint32_t)P.nx * (uint32_t)P.ny;
+            const int l = t.tx * 32 + (int)threadIdx.x;
+            sink.add(l < P.nx && t.m < P.ny ? sweep_column<ZB>(in, out, P, Q.split, l, t.m, t.kb * ZB) : 0u,
+                     P.base + (uint32_t)(t.kb * ZB) * plane + (uint32_t)t.m * (uint32_t)P.nx + (uint32_t)l, plane);
+        });
 }
 
 // Bounded wait on phase `parity` of a shared-memory mbarrier (nanoseconds
@@ -1338,13 +1385,17 @@ __global__ void __launch_bounds__(512, 3) sweep_kernel_tma(const __grid_constant
         }
     }
     BlockSink<ZB> sink(s_cnt);
+    const uint32_t plane = (uint32_t)P.nx * (uint32_t)P.ny;
+    const uint32_t cell0 = (uint32_t)k0 * plane + (uint32_t)m * (uint32_t)P.nx + (uint32_t)l;
     if (row_ok && staged) {
         if (!T.flags) {
-            sink.add(l < P.nx ? sweep_column_tile<ZB>(tile, rows, in, out, P, Q.split, l, m, k0, l0, m0) : 0u);
+            sink.add(l < P.nx ? sweep_column_tile<ZB>(tile, rows, in, out, P, Q.split, l, m, k0, l0, m0) : 0u,
+                     cell0, plane);
         } else if (quiet) {
             if (threadIdx.x == 0) fout[t] = 1;
         } else {
-            sink.add(l < P.nx ? sweep_column_tile<ZB>(tile, rows, in, out, P, Q.split, l, m, k0, l0, m0) : 0u);
+            sink.add(l < P.nx ? sweep_column_tile<ZB>(tile, rows, in, out, P, Q.split, l, m, k0, l0, m0) : 0u,
+                     cell0, plane);
             const bool all = __all_sync(0xffffffffu, sink.codes == 0u);
             if (threadIdx.x == 0) fout[t] = all ? 1 : 0;
         }
@@ -1358,9 +1409,7 @@ __global__ void __launch_bounds__(512, 3) sweep_kernel_tma(const __grid_constant
         s_base[tlin] = n ? atomicAdd(ctr, n) : 0u;
     }
     __syncthreads();
-    if (l < P.nx && m < P.ny && k0 < P.nz)
-        sink.flush(Q, P.cells32, s_base, (uint32_t)P.nx * (uint32_t)P.ny, (uint32_t)m * (uint32_t)P.nx + (uint32_t)l,
-                   k0);
+    sink.flush(Q, P.cells32, s_base);
 }
 
 // The work lists: 0 at items[0..), 1 at items[cells-1..] downwards, 2 at
@@ -1479,7 +1528,7 @@ __global__ void __launch_bounds__(128, 4) trio_kernel(In in, Out out, Mats M, Pa
 
 // list 0: grain boundaries and junctions, beside the above
 template <int S>
-__global__ void __launch_bounds__(256, 3) general_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity) {
+__global__ void __launch_bounds__(256, 4) general_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity) {
     const uint32_t n = *(volatile uint32_t *)(Q.count + 2 * parity);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t c = Q.items[i];
@@ -1626,78 +1675,61 @@ __device__ __forceinline__ Params instance_params(const Params &P0, const mpf3d_
     return P;
 }
 
-// The batched sweep.  One block is one 32 x 8 x SWEEP_ZB tile of one
-// instance, and each of its 8 warps one 32 x 1 x SWEEP_ZB warp tile, whose
-// index is blockIdx.x * 8 + threadIdx.y.  With `flags` (2 x 8 x n_tiles
-// bytes, halves alternating with the step parity; NULL: every tile visited)
-// a warp tile that was uniform in the previous step together with its 6 face
-// neighbours in the same instance (periodic x and y, clamped z) is quiet and
-// skipped, by the argument of the single-domain sweep's quiet tiles.
-template <int S, int AMAX>
-__global__ void __launch_bounds__(256) batched_sweep_kernel(In in, Out out, Params P0,
-                                                            const mpf3d_instance *__restrict__ inst, int n_inst,
-                                                            Queue Q, int parity, uint8_t *__restrict__ flags) {
-    __shared__ uint32_t s_cnt[3], s_base[3];
-    const int tlin = threadIdx.x + 32 * threadIdx.y;
-    if (tlin < 3) s_cnt[tlin] = 0;
-    if (blockIdx.x == 0 && threadIdx.x < 2 && threadIdx.y == 0) Q.count[2 * (parity ^ 1) + threadIdx.x] = 0;
-    if (blockIdx.x == 0 && threadIdx.x == 2 && threadIdx.y == 0 && Q.split) Q.count[4 + (parity ^ 1)] = 0;
-    __syncthreads();
-    // one block is one tile of one instance
-    const int i = find_instance_by_tile(inst, n_inst, (int)blockIdx.x);
-    const mpf3d_instance I = inst[i];
-    const int t = (int)blockIdx.x - I.tile_start;
-    const int tx = (I.nx + 31) / 32, ty = (I.ny + 7) / 8, tz = (I.nz + SWEEP_ZB - 1) / SWEEP_ZB;
-    const int bx = t % tx, kb = t / (tx * ty);
-    const int l = bx * 32 + threadIdx.x;
-    const int m = ((t / tx) % ty) * 8 + threadIdx.y;
-    const int k0 = kb * SWEEP_ZB;
-    const bool row_in = m < I.ny && k0 < I.nz;  // the same for the 32 lanes of a warp
-    const bool inside = l < I.nx && row_in;
-    const Params P = instance_params(P0, I);
-    BlockSink<SWEEP_ZB> sink(s_cnt);
-    if (!flags) {
-        if (row_in) sink.add(inside ? sweep_column(in, out, P, Q.split, l, m, k0) : 0u);
-    } else {
-        const uint32_t nw = gridDim.x * 8u;
-        const uint8_t *fin = flags + (size_t)(parity ^ 1) * nw;
-        uint8_t *fout = flags + (size_t)parity * nw;
-        const uint32_t w = blockIdx.x * 8u + threadIdx.y;
-        const bool lane0 = threadIdx.x == 0;
-        if (!row_in) {
-            if (lane0) fout[w] = 1;
-        } else {
-            // warp tile (x tile a, row mm, z tile c) of this instance
-            auto wt = [&](int a, int mm, int c) {
-                return (uint32_t)(I.tile_start + (c * ty + mm / 8) * tx + a) * 8u + (uint32_t)(mm % 8);
-            };
+// The batched sweep.  An instance is cut into tiles of 32 x 8 x SWEEP_ZB cells
+// (tile_start) and each of those into 8 warp tiles of 32 x 1 x SWEEP_ZB, numbered
+// 8 * tile + row.  With `flags` (2 x 8 x n_tiles bytes, halves alternating with
+// the step parity; NULL: every tile visited) a warp tile that was uniform in the
+// previous step together with its 6 face neighbours in the same instance
+// (periodic x and y, clamped z) is quiet and skipped, by the argument of the
+// single-domain sweep's quiet tiles.
+struct WarpTile {
+    int tile_start, tx, ty, tz, bx, m, kb;
+    __device__ __forceinline__ WarpTile(const mpf3d_instance &I, uint32_t tile, uint32_t row) {
+        tile_start = I.tile_start;
+        tx = (I.nx + 31) / 32, ty = (I.ny + 7) / 8, tz = (I.nz + SWEEP_ZB - 1) / SWEEP_ZB;
+        const int t = (int)tile - tile_start, q = t / tx;
+        bx = t - q * tx, kb = q / ty, m = (q - kb * ty) * 8 + (int)row;
+    }
+    // the number of (x tile, row, z tile) in this instance
+    __device__ __forceinline__ uint32_t at(int a, int mm, int c) const {
+        return (uint32_t)(tile_start + (c * ty + mm / 8) * tx + a) * 8u + (uint32_t)(mm % 8);
+    }
+};
+
+__global__ void __launch_bounds__(256, 6) batched_sweep_kernel(In in, Out out, Params P0,
+                                                               const mpf3d_instance *__restrict__ inst, int n_inst,
+                                                               Queue Q, int parity, uint8_t *__restrict__ flags,
+                                                               uint32_t n_tiles) {
+    if (blockIdx.x == 0) clear_counters(Q, parity, threadIdx.x + 32u * threadIdx.y);
+    const uint8_t *fin = flags + (size_t)(parity ^ 1) * 8 * n_tiles;
+    uint8_t *fout = flags ? flags + (size_t)parity * 8 * n_tiles : nullptr;
+    sweep_tiles<SWEEP_ZB>(
+        Q, P0.cells32, parity, n_tiles, fout, [](uint32_t tile, uint32_t row) { return tile * 8u + row; },
+        [&](uint32_t tile, uint32_t row) {
+            if (!flags) return false;
+            const mpf3d_instance &I = inst[find_instance_by_tile(inst, n_inst, (int)tile)];
+            const WarpTile t(I, tile, row);
+            const int bx = t.bx, m = t.m, kb = t.kb;
+            if (m >= I.ny) return true;  // a row past the instance's top
             // the 7 flags are loaded together (no short-circuit chain of loads)
-            const uint32_t f0 = fin[w];
-            const uint32_t f1 = fin[wt(bx + 1 < tx ? bx + 1 : 0, m, kb)];
-            const uint32_t f2 = fin[wt(bx > 0 ? bx - 1 : tx - 1, m, kb)];
-            const uint32_t f3 = fin[wt(bx, m + 1 < I.ny ? m + 1 : 0, kb)];
-            const uint32_t f4 = fin[wt(bx, m > 0 ? m - 1 : I.ny - 1, kb)];
-            const uint32_t f5 = fin[wt(bx, m, kb + 1 < tz ? kb + 1 : kb)];
-            const uint32_t f6 = fin[wt(bx, m, kb > 0 ? kb - 1 : kb)];
-            if ((f0 & f1 & f2 & f3 & f4 & f5 & f6) != 0u) {
-                if (lane0) fout[w] = 1;
-            } else {
-                sink.add(inside ? sweep_column(in, out, P, Q.split, l, m, k0) : 0u);
-                const bool all = __all_sync(0xffffffffu, sink.codes == 0u);
-                if (lane0) fout[w] = all ? 1 : 0;
-            }
-        }
-    }
-    __syncthreads();
-    if (tlin < 3) {
-        const uint32_t n = s_cnt[tlin];
-        uint32_t *ctr = tlin == 2 ? Q.count + 4 + parity : Q.count + 2 * parity + tlin;
-        s_base[tlin] = n ? atomicAdd(ctr, n) : 0u;
-    }
-    __syncthreads();
-    if (inside)
-        sink.flush(Q, P.cells32, s_base, (uint32_t)P.nx * (uint32_t)P.ny,
-                   P.base + (uint32_t)m * (uint32_t)P.nx + (uint32_t)l, k0);
+            const uint32_t f0 = fin[tile * 8u + row];
+            const uint32_t f1 = fin[t.at(bx + 1 < t.tx ? bx + 1 : 0, m, kb)];
+            const uint32_t f2 = fin[t.at(bx > 0 ? bx - 1 : t.tx - 1, m, kb)];
+            const uint32_t f3 = fin[t.at(bx, m + 1 < I.ny ? m + 1 : 0, kb)];
+            const uint32_t f4 = fin[t.at(bx, m > 0 ? m - 1 : I.ny - 1, kb)];
+            const uint32_t f5 = fin[t.at(bx, m, kb + 1 < t.tz ? kb + 1 : kb)];
+            const uint32_t f6 = fin[t.at(bx, m, kb > 0 ? kb - 1 : kb)];
+            return (f0 & f1 & f2 & f3 & f4 & f5 & f6) != 0u;
+        },
+        [&](uint32_t tile, uint32_t row, BlockSink<SWEEP_ZB> &sink) {
+            const mpf3d_instance I = inst[find_instance_by_tile(inst, n_inst, (int)tile)];
+            const WarpTile t(I, tile, row);
+            const Params P = instance_params(P0, I);
+            const uint32_t plane = (uint32_t)I.nx * (uint32_t)I.ny;
+            const int l = t.bx * 32 + (int)threadIdx.x, k0 = t.kb * SWEEP_ZB;
+            sink.add(l < I.nx && t.m < I.ny ? sweep_column(in, out, P, Q.split, l, t.m, k0) : 0u,
+                     P.base + (uint32_t)k0 * plane + (uint32_t)t.m * (uint32_t)I.nx + (uint32_t)l, plane);
+        });
 }
 
 // The work-list kernels of a batch: as the single domain's, on the instance of
@@ -1742,7 +1774,7 @@ __global__ void __launch_bounds__(128, 4) batched_trio_kernel(In in, Out out, Ma
 
 // list 0: grain boundaries and junctions, beside the above
 template <int S>
-__global__ void __launch_bounds__(256, 3) batched_general_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity) {
+__global__ void __launch_bounds__(256, 4) batched_general_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity) {
     const uint32_t n = *(volatile uint32_t *)(Q.count + 2 * parity);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t c = Q.items[i];
@@ -1969,6 +2001,17 @@ bool side_ready(SideStream &side, cudaStream_t s) {
     return side.ready;
 }
 
+// Blocks of the sweep of `chunks` chunks of `rows` tiles, a warp per row, 48 warps
+// resident per SM: a block per chunk up to SWEEP_WAVES waves of blocks, then up to
+// SWEEP_TILES tiles per block.  (256^3: 23.5 us with 1 wave, 22.7 with 4, 28.4 with
+// 8.)
+constexpr uint32_t SWEEP_WAVES = 4;
+uint32_t sweep_blocks(uint32_t chunks, int rows, int sms) {
+    const uint32_t each = chunks / (SWEEP_WAVES * (uint32_t)sms * 48u / (uint32_t)rows);
+    const uint32_t n = min(max(each, 1u), SWEEP_TILES / (uint32_t)rows);
+    return (chunks + n - 1u) / n;
+}
+
 // Cells from which a step's lists go to pair_kernel, trio_kernel and
 // general_kernel, and what they leave to rest_kernel; on smaller domains the
 // octets take everything.  us per step by octets / by kind, with one grain per
@@ -2033,7 +2076,7 @@ bool head_map(CUtensorMap *map, const uint32_t *head, int nx, int ny, int nz, in
 template <int S, int AMAX>
 void launch_step(const In &in, const Out &out, const Mats &M, const Params &P, const Queue &Q, int parity,
                  uint8_t *tile_flags, int32_t *err, cudaStream_t s, const mpf3d_tuning &T, bool sweep_tma) {
-    const int by = T.sweep_by;
+    const int by = T.sweep_by, sms = sms_of_current_device();
     dim3 blk(32, by, 1);
     CUtensorMap map;
     const bool tma = sweep_tma && P.base == 0 && head_map(&map, in.head, P.nx, P.ny, P.nz, by, T.sweep_zb);
@@ -2042,15 +2085,15 @@ void launch_step(const In &in, const Out &out, const Mats &M, const Params &P, c
         const dim3 grid((P.nx + 31) / 32, (P.ny + by - 1) / by, (P.nz + ZB - 1) / ZB);                             \
         const Tiles tl{tile_flags, (P.nx + 31) / 32, (P.nz + ZB - 1) / ZB, tiles_of<ZB>(P.nx, P.ny, P.nz)};       \
         if (tma) sweep_kernel_tma<S, AMAX, ZB><<<grid, blk, 0, s>>>(map, in, out, P, Q, parity, tl, err);          \
-        else sweep_kernel<S, AMAX, ZB><<<grid, blk, 0, s>>>(in, out, M, P, Q, parity, tl, err);                    \
+        else {                                                                                                     \
+            const uint32_t chunks = grid.x * grid.y * grid.z;                                                      \
+            sweep_kernel<ZB><<<sweep_blocks(chunks, by, sms), blk, 0, s>>>(in, out, P, Q, parity, tl, chunks);     \
+        }                                                                                                          \
     } while (0)
     if (T.sweep_zb == 2) SWEEP_LAUNCH(2);
     else if (T.sweep_zb == 8) SWEEP_LAUNCH(8);
     else SWEEP_LAUNCH(4);
 #undef SWEEP_LAUNCH
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (P.cells < PAIR_CELLS) {  // 8 blocks of 128 threads are resident per SM
         if (P.sym_normals) octet_kernel<S, AMAX, 4><<<sms * 8, 128, 0, s>>>(in, out, M, P, Q, parity, err);
         else octet_kernel<S, AMAX, 8><<<sms * 8, 128, 0, s>>>(in, out, M, P, Q, parity, err);
@@ -2216,12 +2259,12 @@ template <int S, int AMAX>
 void launch_batched(const In &in, const Out &out, const Mats &M, const Params &P0, const mpf3d_instance *inst,
                     int n_inst, int n_tiles, const Queue &Q, int parity, int32_t *err, cudaStream_t s,
                     const mpf3d_tuning &T, uint8_t *tile_flags) {
-    batched_sweep_kernel<S, AMAX><<<n_tiles, dim3(32, 8, 1), 0, s>>>(in, out, P0, inst, n_inst, Q, parity,
-                                                                      tile_flags);
+    const int sms = sms_of_current_device();
+    batched_sweep_kernel<<<sweep_blocks((uint32_t)n_tiles, 8, sms), dim3(32, 8, 1), 0, s>>>(
+        in, out, P0, inst, n_inst, Q, parity, tile_flags, (uint32_t)n_tiles);
     // one stream: the side-by-side launch of the compact step measured no
     // gain here; the work-list grids come from T (the sweep's 32 x 8 x 4
     // tiles are fixed by the instance table)
-    const int sms = sms_of_current_device();
     const int g_iface = sms * T.iface_blocks_per_sm, g_general = sms * T.general_blocks_per_sm;
     if (P0.cells < PAIR_CELLS) {  // as the single domain's step
         if (P0.sym_normals)
