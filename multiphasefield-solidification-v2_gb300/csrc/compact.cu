@@ -171,8 +171,8 @@ __device__ __forceinline__ uint32_t cidx(const Params &P, int l, int m, int k) {
 __device__ __forceinline__ float liquid32(const In &in, uint32_t q) {
     const uint32_t h = __ldg(in.head + q);
     const float v = __ldg(in.val + q);
-    if (hcount(h) == 0 || hid0(h) != LIQ) return 0.0f;
-    return (hcount(h) >= 2 || hexplicit(h)) ? v : 1.0f;
+    // a head with liquid is 1..255, alone and implicit 1
+    return h - 1u < 255u ? (h == 1u ? 1.0f : v) : 0.0f;
 }
 
 // 7-point Laplacian of one phase, rounded operation by operation
@@ -190,6 +190,19 @@ __device__ __forceinline__ float lap7(const Params &P, const float (&v)[7]) {
 // and both forms of the interface update, give the same bits.
 __device__ __forceinline__ float dot3(float a, float b, float c, float x, float y, float z) {
     return fmaf(a, x, fmaf(b, y, __fmul_rn(c, z)));
+}
+
+// sqrtf and __fdividef as this file is compiled (-prec-sqrt=false), for normal
+// numbers: without the scaling of subnormal ones
+__device__ __forceinline__ float root(float x) {
+    float y;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float ratio(float a, float b) {
+    float y;
+    asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+    return y;
 }
 
 // The liquid gradient (or the dominant solid's) at a stencil point.
@@ -216,23 +229,22 @@ struct PointTerms {
 template <int NT>
 __device__ __forceinline__ PointTerms point_terms(const Params &P, const Grad &G, const float (&un)[3 * NT]) {
     PointTerms t;
-    t.cabs = 0.0f; t.cs = 0.0f; t.nx = 1.0f; t.ny = 0.0f; t.nz = 0.0f;
+    t.cs = 0.0f; t.nx = 1.0f; t.ny = 0.0f; t.nz = 0.0f;
     const float x = G.g.x * G.ig, y = G.g.y * G.ig, z = G.g.z * G.ig;
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
         const float d = dot3(x, y, z, un[3 * i], un[3 * i + 1], un[3 * i + 2]);
-        const float a = fabsf(d);
-        if (a > t.cabs) {
-            t.cabs = a; t.cs = d; t.nx = un[3 * i]; t.ny = un[3 * i + 1]; t.nz = un[3 * i + 2];
+        if (fabsf(d) > fabsf(t.cs)) {
+            t.cs = d; t.nx = un[3 * i]; t.ny = un[3 * i + 1]; t.nz = un[3 * i + 2];
         }
     }
-    t.cabs = fminf(t.cabs, 1.0f);
+    t.cabs = fminf(fabsf(t.cs), 1.0f);
     t.cs = fminf(fmaxf(t.cs, -1.0f), 1.0f);
-    const float C = sqrtf(fmaf(t.cs, t.cs, P.pp)), Sn = sqrtf(fmaxf(fmaf(-t.cs, t.cs, 1.0f), 0.0f) + P.pp);
+    const float C = root(fmaf(t.cs, t.cs, P.pp)), Sn = root(fmaxf(fmaf(-t.cs, t.cs, 1.0f), 0.0f) + P.pp);
     t.a = P.mu_a * fmaf(P.delta_a, fmaf(P.tan_a0, Sn, C), 1.0f);
     const float e = P.eps0 * t.a;
     t.e2 = G.valid ? e * e : P.e2_flat;
-    t.coef = P.mu_da * fmaf(-P.tan_a0, __fdividef(t.cs, Sn), __fdividef(t.cs, C));
+    t.coef = P.mu_da * fmaf(-P.tan_a0, ratio(t.cs, Sn), ratio(t.cs, C));
     return t;
 }
 // d cos / d(grad phi); 0 below the floor
@@ -283,27 +295,40 @@ __device__ __forceinline__ float arm_sum(const float (&f)[7]) {
     return __fadd_rn(__fadd_rn(f[1], __fadd_rn(f[2], f[3])), __fadd_rn(__fadd_rn(f[4], f[5]), f[6]));
 }
 
+// Cell (l, m, k) and the steps to its neighbours in cell indices, modulo 2^32
+// (x and y periodic, z clamped): one step each way, and two.
+struct Offsets {
+    uint32_t c, xp, xm, yp, ym, zp, zm, x2p, x2m, y2p, y2m, z2p, z2m;
+    __device__ __forceinline__ Offsets(const Params &P, int l, int m, int k) {
+        c = cidx(P, l, m, k);
+        const uint32_t nx = (uint32_t)P.nx, plane = nx * (uint32_t)P.ny;
+        const int lp = wrap_p(l, P.nx), lm = wrap_m(l, P.nx), mp = wrap_p(m, P.ny), mm = wrap_m(m, P.ny);
+        xp = (uint32_t)(lp - l), xm = (uint32_t)(lm - l);
+        x2p = (uint32_t)(wrap_p(lp, P.nx) - l), x2m = (uint32_t)(wrap_m(lm, P.nx) - l);
+        yp = (uint32_t)(mp - m) * nx, ym = (uint32_t)(mm - m) * nx;
+        y2p = (uint32_t)(wrap_p(mp, P.ny) - m) * nx, y2m = (uint32_t)(wrap_m(mm, P.ny) - m) * nx;
+        zp = k < P.nz - 1 ? plane : 0u, zm = k > 0 ? 0u - plane : 0u;
+        z2p = k < P.nz - 2 ? 2u * plane : zp, z2m = k > 1 ? 0u - 2u * plane : zm;
+    }
+};
+
 // Liquid gradients at the 7 points and mixed second differences at the cell,
 // from the liquid vL there and at the 18 further points of the 25-point stencil
 // (offsets with |dx|+|dy|+|dz| <= 2).
 struct Stencil {
     float3 G[7];
     float hxy, hxz, hyz;
-    __device__ __forceinline__ Stencil(const In &in, const Params &P, int l, int m, int k, const float (&vL)[7]) {
-        const int lp = wrap_p(l, P.nx), lm = wrap_m(l, P.nx), mp = wrap_p(m, P.ny), mm = wrap_m(m, P.ny);
-        const int kp = clamp_p(k, P.nz), km = clamp_m(k, P.nz);
-        const int lpp = wrap_p(lp, P.nx), lmm = wrap_m(lm, P.nx);
-        const int mpp = wrap_p(mp, P.ny), mmm = wrap_m(mm, P.ny);
-        const int kpp = clamp_p(kp, P.nz), kmm = clamp_m(km, P.nz);
-        const float Lxpyp = liquid32(in, cidx(P, lp, mp, k)), Lxpym = liquid32(in, cidx(P, lp, mm, k));
-        const float Lxmyp = liquid32(in, cidx(P, lm, mp, k)), Lxmym = liquid32(in, cidx(P, lm, mm, k));
-        const float Lxpzp = liquid32(in, cidx(P, lp, m, kp)), Lxpzm = liquid32(in, cidx(P, lp, m, km));
-        const float Lxmzp = liquid32(in, cidx(P, lm, m, kp)), Lxmzm = liquid32(in, cidx(P, lm, m, km));
-        const float Lypzp = liquid32(in, cidx(P, l, mp, kp)), Lypzm = liquid32(in, cidx(P, l, mp, km));
-        const float Lymzp = liquid32(in, cidx(P, l, mm, kp)), Lymzm = liquid32(in, cidx(P, l, mm, km));
-        const float Lx2p = liquid32(in, cidx(P, lpp, m, k)), Lx2m = liquid32(in, cidx(P, lmm, m, k));
-        const float Ly2p = liquid32(in, cidx(P, l, mpp, k)), Ly2m = liquid32(in, cidx(P, l, mmm, k));
-        const float Lz2p = liquid32(in, cidx(P, l, m, kpp)), Lz2m = liquid32(in, cidx(P, l, m, kmm));
+    __device__ __forceinline__ Stencil(const In &in, const Params &P, const Offsets &o, const float (&vL)[7]) {
+        const float Lxpyp = liquid32(in, o.c + o.xp + o.yp), Lxpym = liquid32(in, o.c + o.xp + o.ym);
+        const float Lxmyp = liquid32(in, o.c + o.xm + o.yp), Lxmym = liquid32(in, o.c + o.xm + o.ym);
+        const float Lxpzp = liquid32(in, o.c + o.xp + o.zp), Lxpzm = liquid32(in, o.c + o.xp + o.zm);
+        const float Lxmzp = liquid32(in, o.c + o.xm + o.zp), Lxmzm = liquid32(in, o.c + o.xm + o.zm);
+        const float Lypzp = liquid32(in, o.c + o.yp + o.zp), Lypzm = liquid32(in, o.c + o.yp + o.zm);
+        const float Lymzp = liquid32(in, o.c + o.ym + o.zp), Lymzm = liquid32(in, o.c + o.ym + o.zm);
+        const float Lx2p = liquid32(in, o.c + o.x2p), Lx2m = liquid32(in, o.c + o.x2m);
+        const float Ly2p = liquid32(in, o.c + o.y2p), Ly2m = liquid32(in, o.c + o.y2m);
+        const float Lz2p = liquid32(in, o.c + o.z2p), Lz2m = liquid32(in, o.c + o.z2m);
+        const bool top = o.zp == 0, bottom = o.zm == 0;
         const float g2 = P.inv_2dx;
         G[0] = make_float3((vL[1] - vL[2]) * g2, (vL[3] - vL[4]) * g2, (vL[5] - vL[6]) * g2);
         G[1] = make_float3((Lx2p - vL[0]) * g2, (Lxpyp - Lxpym) * g2, (Lxpzp - Lxpzm) * g2);
@@ -312,10 +337,10 @@ struct Stencil {
         G[4] = make_float3((Lxpym - Lxmym) * g2, (vL[0] - Ly2m) * g2, (Lymzp - Lymzm) * g2);
         // z neighbours sit on the clamped rows: at the top/bottom row the
         // neighbour is the cell itself
-        G[5] = (kp == k) ? G[0] : make_float3((Lxpzp - Lxmzp) * g2, (Lypzp - Lymzp) * g2, (Lz2p - vL[0]) * g2);
-        G[6] = (km == k) ? G[0] : make_float3((Lxpzm - Lxmzm) * g2, (Lypzm - Lymzm) * g2, (vL[0] - Lz2m) * g2);
-        if (kp == k) G[5].z = (vL[5] - vL[6]) * g2;
-        if (km == k) G[6].z = (vL[5] - vL[6]) * g2;
+        G[5] = (top) ? G[0] : make_float3((Lxpzp - Lxmzp) * g2, (Lypzp - Lymzp) * g2, (Lz2p - vL[0]) * g2);
+        G[6] = (bottom) ? G[0] : make_float3((Lxpzm - Lxmzm) * g2, (Lypzm - Lymzm) * g2, (vL[0] - Lz2m) * g2);
+        if (top) G[5].z = (vL[5] - vL[6]) * g2;
+        if (bottom) G[6].z = (vL[5] - vL[6]) * g2;
         hxy = (Lxpyp - Lxpym) - (Lxmyp - Lxmym);
         hxz = (Lxpzp - Lxpzm) - (Lxmzp - Lxmzm);
         hyz = (Lypzp - Lypzm) - (Lymzp - Lymzm);
@@ -368,17 +393,14 @@ __device__ __forceinline__ void interface_terms(const Params &P, const Stencil &
 // memory, the two list kernels took 150 us.  By octets alone the lists take 292.
 
 // Update of an interface cell whose neighbourhood holds the liquid and one
-// solid (list 1 where the sweep split the lists): no merge, and only the pair's
-// terms.  Returns false, with nothing written, where the neighbourhood holds
-// more.
+// solid, as the sweep's list 1 does where it split the lists: no merge, and only
+// the pair's terms.
 template <int NT>
-__device__ __forceinline__ bool pair_cell(const In &in, const Out &out, const Mats &M, const Params &P, int l, int m,
+__device__ __forceinline__ void pair_cell(const In &in, const Out &out, const Mats &M, const Params &P, int l, int m,
                                           int k) {
     const uint32_t cells = P.cells32;
-    const int lp = wrap_p(l, P.nx), lm = wrap_m(l, P.nx), mp = wrap_p(m, P.ny), mm = wrap_m(m, P.ny);
-    const int kp = clamp_p(k, P.nz), km = clamp_m(k, P.nz);
-    const uint32_t pt[7] = {cidx(P, l, m, k), cidx(P, lp, m, k), cidx(P, lm, m, k), cidx(P, l, mp, k),
-                            cidx(P, l, mm, k), cidx(P, l, m, kp), cidx(P, l, m, km)};
+    const Offsets at(P, l, m, k);
+    const uint32_t pt[7] = {at.c, at.c + at.xp, at.c + at.xm, at.c + at.yp, at.c + at.ym, at.c + at.zp, at.c + at.zm};
     uint32_t h[7];
     float v0[7], v1[7];
     int i1[7];
@@ -389,21 +411,18 @@ __device__ __forceinline__ bool pair_cell(const In &in, const Out &out, const Ma
         i1[p] = (int)__ldg(in.idx + cells + pt[p]);
         v1[p] = __ldg(in.val + cells + pt[p]);
     }
+    // heads: none 0; liquid 1 or explicit 0x81; liquid and solid 2; solid id << 8
+    // | 1 or explicit
     float vL[7], vS[7];
     int sid = 0;
-    bool pair = true;
 #pragma unroll
     for (int p = 0; p < 7; ++p) {
-        const int n = hcount(h[p]), id = hid0(h[p]);
-        const float v = n >= 2 || hexplicit(h[p]) ? v0[p] : 1.0f;
-        vL[p] = n >= 1 && id == LIQ ? v : 0.0f;
-        vS[p] = n >= 2 ? v1[p] : (n == 1 && id != LIQ ? v : 0.0f);
-        const int s = n >= 2 ? i1[p] : (n == 1 ? id : LIQ);  // the point's solid, LIQ for none
-        pair = pair && (n < 2 || (n == 2 && id == LIQ)) && (s == LIQ || sid == 0 || s == sid);
-        sid = s != LIQ ? s : sid;
+        const float v = (h[p] & 0xffu) == 1u ? 1.0f : v0[p];
+        vL[p] = h[p] - 1u < 255u ? v : 0.0f;
+        vS[p] = h[p] == 2u ? v1[p] : (h[p] > 255u ? v : 0.0f);
+        sid = max(sid, h[p] == 2u ? i1[p] : hid0(h[p]));
     }
-    if (!pair || sid == 0) return false;
-    const Stencil st(in, P, l, m, k, vL);
+    const Stencil st(in, P, at, vL);
     const float *ug = M.n111 + (size_t)(P.n111_base + sid) * 24;
     float un[3 * NT], lap_sl, b_sl;
 #pragma unroll
@@ -442,7 +461,6 @@ __device__ __forceinline__ bool pair_cell(const In &in, const Out &out, const Ma
         out.val[cells + c] = rS;
     }
     out.head[c] = mkhead(keepL || !keepS ? LIQ : sid, (keepL ? 1 : 0) + (keepS ? 1 : 0), false);
-    return true;
 }
 
 // Update of a cell whose neighbourhood holds up to three phases, in registers:
@@ -512,7 +530,7 @@ __device__ __forceinline__ bool trio_cell(const In &in, const Out &out, const Ma
     float w_sl = P.w0;
     if (ids[0] == LIQ && n > 1) {
         if (HEAVY) {
-            const Stencil st(in, P, l, m, k, V[0]);
+            const Stencil st(in, P, Offsets(P, l, m, k), V[0]);
             // dominant solid
             const bool last = n == 3 && V[2][0] > V[1][0];
             const float3 gs = last ? make_float3((V[2][1] - V[2][2]) * P.inv_2dx, (V[2][3] - V[2][4]) * P.inv_2dx,
@@ -1148,17 +1166,19 @@ __device__ __forceinline__ void advance_clock(const Params &P) {
 // gridDim.x-th chunk, at most SWEEP_TILES tiles (distant ones: the tiles that are
 // not quiet lie together).  A lane per tile reads its flags (quiet), then the warps
 // share the others, one per warp and round; visit fills the warp's sink, flag_of
-// is a tile's place in fout.  A warp of its own for each of the 79 % quiet tiles of
+// is a tile's place in fout, domain_of a chunk's instance.  A warp of its own for each of the 79 % quiet tiles of
 // a 256^3 step with 64 grains spent the time on starting blocks; us per step with a
 // block per chunk / with up to 128 tiles per block: 256^3 41 / 23, 512 x 512 x 256
 // 155 / 63 (64 tiles: 69, 32: 78), 24 bicrystals 92 / 79.  With consecutive chunks
 // per block, 256^3 took 43: blocks whose tiles are all visited came last.
 constexpr uint32_t SWEEP_TILES = 128;  // blocks have at least as many threads
 
-template <int ZB, class Flag, class Quiet, class Visit>
+template <int ZB, class Domain, class Flag, class Quiet, class Visit>
 __device__ __forceinline__ void sweep_tiles(const Queue &Q, uint32_t cells, int parity, uint32_t chunks,
-                                            uint8_t *__restrict__ fout, Flag &&flag_of, Quiet &&quiet, Visit &&visit) {
+                                            uint8_t *__restrict__ fout, Domain &&domain_of, Flag &&flag_of,
+                                            Quiet &&quiet, Visit &&visit) {
     __shared__ uint32_t s_cnt[3], s_base[3], s_tile[SWEEP_TILES], s_n;
+    __shared__ int s_of[SWEEP_TILES];
     const uint32_t lane = threadIdx.x, tlin = lane + 32u * threadIdx.y, rows = blockDim.y;
     if (tlin < 3) s_cnt[tlin] = 0;
     if (tlin == 3) s_n = 0;
@@ -1166,13 +1186,18 @@ __device__ __forceinline__ void sweep_tiles(const Queue &Q, uint32_t cells, int 
     if (32u * threadIdx.y < SWEEP_TILES) {
         const uint32_t chunk = blockIdx.x + tlin / rows * gridDim.x, row = tlin % rows;
         const bool in = chunk < chunks;
-        const bool skip = in && quiet(chunk, row);
+        const int of = in ? domain_of(chunk) : 0;
+        const bool skip = in && quiet(of, chunk, row);
         if (skip && fout) fout[flag_of(chunk, row)] = 1;
         const unsigned mask = __ballot_sync(0xffffffffu, in && !skip);
         uint32_t at = 0;
         if (lane == 0 && mask) at = atomicAdd(&s_n, (uint32_t)__popc(mask));
         at = __shfl_sync(0xffffffffu, at, 0);
-        if (mask >> lane & 1u) s_tile[at + __popc(mask & ((1u << lane) - 1u))] = chunk * rows + row;
+        at += __popc(mask & ((1u << lane) - 1u));
+        if (mask >> lane & 1u) {
+            s_tile[at] = chunk * rows + row;
+            s_of[at] = of;
+        }
     }
     __syncthreads();
     const uint32_t n = s_n;
@@ -1180,7 +1205,7 @@ __device__ __forceinline__ void sweep_tiles(const Queue &Q, uint32_t cells, int 
         BlockSink<ZB> sink(s_cnt);
         if (r + threadIdx.y < n) {
             const uint32_t t = s_tile[r + threadIdx.y], chunk = t / rows, row = t - chunk * rows;
-            visit(chunk, row, sink);
+            visit(s_of[r + threadIdx.y], chunk, row, sink);
             if (fout) {
                 const bool all = __all_sync(0xffffffffu, sink.codes == 0u);
                 if (lane == 0) fout[flag_of(chunk, row)] = all ? 1 : 0;
@@ -1226,12 +1251,12 @@ __global__ void __launch_bounds__(512, 3) sweep_kernel(In in, Out out, Params P,
     };
     auto at = [&](int a, int b, int c) { return ((uint32_t)c * (uint32_t)P.ny + (uint32_t)b) * ntx + (uint32_t)a; };
     sweep_tiles<ZB>(
-        Q, P.cells32, parity, chunks, fout,
+        Q, P.cells32, parity, chunks, fout, [](uint32_t) { return 0; },
         [&](uint32_t chunk, uint32_t row) {
             const Tile t = tile_of(chunk, row);
             return at(t.tx, t.m, t.kb);
         },
-        [&](uint32_t chunk, uint32_t row) {
+        [&](int, uint32_t chunk, uint32_t row) {
             const auto [tx, m, kb] = tile_of(chunk, row);
             if (!T.flags || m >= P.ny) return false;
             // the 7 flags are loaded together (no short-circuit chain of loads)
@@ -1244,7 +1269,7 @@ __global__ void __launch_bounds__(512, 3) sweep_kernel(In in, Out out, Params P,
             const uint32_t f6 = fin[at(tx, m, kb > 0 ? kb - 1 : kb)];
             return (f0 & f1 & f2 & f3 & f4 & f5 & f6) != 0u;
         },
-        [&](uint32_t chunk, uint32_t row, BlockSink<ZB> &sink) {
+        [&](int, uint32_t chunk, uint32_t row, BlockSink<ZB> &sink) {
             const Tile t = tile_of(chunk, row);
             const uint32_t plane = (uint32_t)P.nx * (uint32_t)P.ny;
             const int l = t.tx * 32 + (int)threadIdx.x;
@@ -1696,7 +1721,7 @@ struct WarpTile {
     }
 };
 
-__global__ void __launch_bounds__(256, 6) batched_sweep_kernel(In in, Out out, Params P0,
+__global__ void __launch_bounds__(256, 8) batched_sweep_kernel(In in, Out out, Params P0,
                                                                const mpf3d_instance *__restrict__ inst, int n_inst,
                                                                Queue Q, int parity, uint8_t *__restrict__ flags,
                                                                uint32_t n_tiles) {
@@ -1704,10 +1729,12 @@ __global__ void __launch_bounds__(256, 6) batched_sweep_kernel(In in, Out out, P
     const uint8_t *fin = flags + (size_t)(parity ^ 1) * 8 * n_tiles;
     uint8_t *fout = flags ? flags + (size_t)parity * 8 * n_tiles : nullptr;
     sweep_tiles<SWEEP_ZB>(
-        Q, P0.cells32, parity, n_tiles, fout, [](uint32_t tile, uint32_t row) { return tile * 8u + row; },
-        [&](uint32_t tile, uint32_t row) {
+        Q, P0.cells32, parity, n_tiles, fout,
+        [&](uint32_t tile) { return find_instance_by_tile(inst, n_inst, (int)tile); },
+        [](uint32_t tile, uint32_t row) { return tile * 8u + row; },
+        [&](int i, uint32_t tile, uint32_t row) {
             if (!flags) return false;
-            const mpf3d_instance &I = inst[find_instance_by_tile(inst, n_inst, (int)tile)];
+            const mpf3d_instance &I = inst[i];
             const WarpTile t(I, tile, row);
             const int bx = t.bx, m = t.m, kb = t.kb;
             if (m >= I.ny) return true;  // a row past the instance's top
@@ -1721,8 +1748,8 @@ __global__ void __launch_bounds__(256, 6) batched_sweep_kernel(In in, Out out, P
             const uint32_t f6 = fin[t.at(bx, m, kb > 0 ? kb - 1 : kb)];
             return (f0 & f1 & f2 & f3 & f4 & f5 & f6) != 0u;
         },
-        [&](uint32_t tile, uint32_t row, BlockSink<SWEEP_ZB> &sink) {
-            const mpf3d_instance I = inst[find_instance_by_tile(inst, n_inst, (int)tile)];
+        [&](int i, uint32_t tile, uint32_t row, BlockSink<SWEEP_ZB> &sink) {
+            const mpf3d_instance I = inst[i];
             const WarpTile t(I, tile, row);
             const Params P = instance_params(P0, I);
             const uint32_t plane = (uint32_t)I.nx * (uint32_t)I.ny;
