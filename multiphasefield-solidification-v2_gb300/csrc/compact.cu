@@ -189,7 +189,7 @@ __device__ __forceinline__ float lap7(const Params &P, const float (&v)[7]) {
 // with explicit roundings throughout, so that every kernel that inlines them,
 // and both forms of the interface update, give the same bits.
 __device__ __forceinline__ float dot3(float a, float b, float c, float x, float y, float z) {
-    return fmaf(a, x, fmaf(b, y, __fmul_rn(c, z)));
+    return fmaf(c, z, fmaf(a, x, __fmul_rn(b, y)));
 }
 
 // sqrtf and __fdividef as this file is compiled (-prec-sqrt=false), for normal
