@@ -34,6 +34,7 @@
 
 #include <mutex>
 #include <unordered_map>
+#include <utility>
 
 #include "compact_state.cuh"
 #include "mpf3d.h"
@@ -1223,6 +1224,14 @@ __device__ __forceinline__ void sweep_tiles(const Queue &Q, uint32_t cells, int 
     }
 }
 
+// First statements of a kernel that launch_early starts: its blocks may be
+// resident before the stream's previous kernel is complete, and wait here until
+// it is and its writes are visible; the next such kernel may do the same.
+__device__ __forceinline__ void wait_for_previous() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // the other parity's counters, which the previous step's kernels are done with
 __device__ __forceinline__ void clear_counters(const Queue &Q, int parity, uint32_t t) {
     if (t < 2) Q.count[2 * (parity ^ 1) + t] = 0;
@@ -1234,6 +1243,7 @@ __device__ __forceinline__ void clear_counters(const Queue &Q, int parity, uint3
 template <int ZB>
 __global__ void __launch_bounds__(512, 3) sweep_kernel(In in, Out out, Params P, Queue Q, int parity, Tiles T,
                                                        uint32_t chunks) {
+    wait_for_previous();
     if (blockIdx.x == 0) {
         const uint32_t t = threadIdx.x + 32u * threadIdx.y;
         clear_counters(Q, parity, t);
@@ -1521,6 +1531,7 @@ struct Place {
 template <int S, int AMAX, int NT>
 __global__ void __launch_bounds__(128, 8) octet_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity,
                                                        int32_t *__restrict__ err) {
+    wait_for_previous();
     const OctetLane O;
     for_octets(Q, P.cells32, parity, [&](uint32_t c, bool active) {
         const Place at(c, P.nx, P.ny);
@@ -1542,6 +1553,7 @@ __global__ void __launch_bounds__(128, 5) pair_kernel(In in, Out out, Mats M, Pa
 // list 2: multi-solid interface cells
 template <int S, int NT>
 __global__ void __launch_bounds__(128, 4) trio_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity) {
+    wait_for_previous();
     const uint32_t n = *(volatile uint32_t *)(Q.count + (Q.split ? 4 + parity : 2 * parity + 1));
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t &item = Q.items[Q.split ? P.cells32 + i : P.cells32 - 1u - i];
@@ -1554,6 +1566,7 @@ __global__ void __launch_bounds__(128, 4) trio_kernel(In in, Out out, Mats M, Pa
 // list 0: grain boundaries and junctions, beside the above
 template <int S>
 __global__ void __launch_bounds__(256, 4) general_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity) {
+    wait_for_previous();
     const uint32_t n = *(volatile uint32_t *)(Q.count + 2 * parity);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t c = Q.items[i];
@@ -1566,6 +1579,7 @@ __global__ void __launch_bounds__(256, 4) general_kernel(In in, Out out, Mats M,
 template <int S, int AMAX, int NT>
 __global__ void __launch_bounds__(128, 8)
     rest_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity, int32_t *__restrict__ err) {
+    wait_for_previous();
     const OctetLane O;
     Lists L(Q, parity);
     if (Q.split) L.n[1] = 0;
@@ -1584,6 +1598,7 @@ __global__ void __launch_bounds__(128, 8)
 template <int S, int AMAX>
 __global__ void __launch_bounds__(256, 3)
     isotropic_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity, int32_t *__restrict__ err) {
+    wait_for_previous();
     const OctetLane O;
     for_items<32, 256>(
         *(volatile uint32_t *)(Q.count + 2 * parity), [&](uint32_t i) { return Q.items[i]; },
@@ -1794,6 +1809,7 @@ __global__ void __launch_bounds__(256, 8) batched_sweep_kernel(In in, Out out, P
                                                                const mpf3d_instance *__restrict__ inst, int n_inst,
                                                                Queue Q, int parity, uint8_t *__restrict__ flags,
                                                                uint32_t n_tiles) {
+    wait_for_previous();
     if (blockIdx.x == 0) clear_counters(Q, parity, threadIdx.x + 32u * threadIdx.y);
     const uint8_t *fin = flags + (size_t)(parity ^ 1) * 8 * n_tiles;
     uint8_t *fout = flags ? flags + (size_t)parity * 8 * n_tiles : nullptr;
@@ -1834,6 +1850,7 @@ template <int S, int AMAX, int NT>
 __global__ void __launch_bounds__(128, 8) batched_octet_kernel(In in, Out out, Mats M, Params P0,
                                                                const mpf3d_instance *__restrict__ inst, int n_inst,
                                                                Queue Q, int parity, int32_t *__restrict__ err) {
+    wait_for_previous();
     const OctetLane O;
     for_octets(Q, P0.cells32, parity, [&](uint32_t c, bool active) {
         const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
@@ -1846,6 +1863,7 @@ template <int NT>
 __global__ void __launch_bounds__(128, 5) batched_pair_kernel(In in, Out out, Mats M, Params P0,
                                                               const mpf3d_instance *__restrict__ inst, int n_inst,
                                                               Queue Q, int parity) {
+    wait_for_previous();
     const uint32_t n = *(volatile uint32_t *)(Q.count + 2 * parity + 1);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t c = Q.items[P0.cells32 - 1u - i];
@@ -1858,6 +1876,7 @@ __global__ void __launch_bounds__(128, 5) batched_pair_kernel(In in, Out out, Ma
 // list 2: multi-solid interface cells
 template <int S, int NT>
 __global__ void __launch_bounds__(128, 4) batched_trio_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity) {
+    wait_for_previous();
     const uint32_t n = *(volatile uint32_t *)(Q.count + (Q.split ? 4 + parity : 2 * parity + 1));
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t &item = Q.items[Q.split ? P0.cells32 + i : P0.cells32 - 1u - i];
@@ -1871,6 +1890,7 @@ __global__ void __launch_bounds__(128, 4) batched_trio_kernel(In in, Out out, Ma
 // list 0: grain boundaries and junctions, beside the above
 template <int S>
 __global__ void __launch_bounds__(256, 4) batched_general_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity) {
+    wait_for_previous();
     const uint32_t n = *(volatile uint32_t *)(Q.count + 2 * parity);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t c = Q.items[i];
@@ -1884,6 +1904,7 @@ __global__ void __launch_bounds__(256, 4) batched_general_kernel(In in, Out out,
 template <int S, int AMAX, int NT>
 __global__ void __launch_bounds__(128, 8)
     batched_rest_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity, int32_t *__restrict__ err) {
+    wait_for_previous();
     const OctetLane O;
     Lists L(Q, parity);
     if (Q.split) L.n[1] = 0;
@@ -1903,6 +1924,7 @@ __global__ void __launch_bounds__(128, 8)
 template <int S, int AMAX>
 __global__ void __launch_bounds__(256, 3)
     batched_isotropic_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity, int32_t *__restrict__ err) {
+    wait_for_previous();
     const OctetLane O;
     for_items<32, 256>(
         *(volatile uint32_t *)(Q.count + 2 * parity), [&](uint32_t i) { return Q.items[i]; },
@@ -2195,6 +2217,22 @@ bool head_map(CUtensorMap *map, const uint32_t *head, int nx, int ny, int nz, in
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Launch of a kernel that begins with wait_for_previous, without waiting for the
+// kernel before it in the stream to drain.
+template <class... K, class... A>
+void launch_early(void (*kernel)(K...), unsigned grid, dim3 block, cudaStream_t s, A &&...args) {
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+
 template <int S, int AMAX>
 void launch_step(const In &in, const Out &out, const Mats &M, const Params &P, const Queue &Q, int parity,
                  uint8_t *tile_flags, int32_t *err, cudaStream_t s, const mpf3d_tuning &T, bool sweep_tma) {
@@ -2209,7 +2247,8 @@ void launch_step(const In &in, const Out &out, const Mats &M, const Params &P, c
         if (tma) sweep_kernel_tma<S, AMAX, ZB><<<grid, blk, 0, s>>>(map, in, out, P, Q, parity, tl, err);          \
         else {                                                                                                     \
             const uint32_t chunks = grid.x * grid.y * grid.z;                                                      \
-            sweep_kernel<ZB><<<sweep_blocks(chunks, by, sms), blk, 0, s>>>(in, out, P, Q, parity, tl, chunks);     \
+            launch_early(sweep_kernel<ZB>, sweep_blocks(chunks, by, sms), blk, s, in, out, P, Q, parity, tl,       \
+                         chunks);                                                                                  \
         }                                                                                                          \
     } while (0)
     if (T.sweep_zb == 2) SWEEP_LAUNCH(2);
@@ -2217,21 +2256,21 @@ void launch_step(const In &in, const Out &out, const Mats &M, const Params &P, c
     else SWEEP_LAUNCH(4);
 #undef SWEEP_LAUNCH
     if (P.cells < PAIR_CELLS) {  // 8 blocks of 128 threads are resident per SM
-        if (P.sym_normals) octet_kernel<S, AMAX, 4><<<sms * 8, 128, 0, s>>>(in, out, M, P, Q, parity, err);
-        else octet_kernel<S, AMAX, 8><<<sms * 8, 128, 0, s>>>(in, out, M, P, Q, parity, err);
+        launch_early(P.sym_normals ? octet_kernel<S, AMAX, 4> : octet_kernel<S, AMAX, 8>, sms * 8, dim3(128), s, in,
+                     out, M, P, Q, parity, err);
         return;
     }
     const int g_general = sms * T.general_blocks_per_sm, g_iface = sms * T.iface_blocks_per_sm;
     if (!P.use_aniso) {
-        isotropic_kernel<S, AMAX><<<g_general, T.general_threads, 0, s>>>(in, out, M, P, Q, parity, err);
+        launch_early(isotropic_kernel<S, AMAX>, g_general, dim3(T.general_threads), s, in, out, M, P, Q, parity, err);
         return;
     }
     launch_side_by_side(
         s,
         [&](cudaStream_t st) {
-            if (P.sym_normals) trio_kernel<S, 4><<<g_iface, T.iface_threads, 0, st>>>(in, out, M, P, Q, parity);
-            else trio_kernel<S, 8><<<g_iface, T.iface_threads, 0, st>>>(in, out, M, P, Q, parity);
-            general_kernel<S><<<g_general, T.general_threads, 0, st>>>(in, out, M, P, Q, parity);
+            launch_early(P.sym_normals ? trio_kernel<S, 4> : trio_kernel<S, 8>, g_iface, dim3(T.iface_threads), st, in,
+                         out, M, P, Q, parity);
+            launch_early(general_kernel<S>, g_general, dim3(T.general_threads), st, in, out, M, P, Q, parity);
         },
         [&](cudaStream_t st) {
             if (!Q.split) return;
@@ -2368,34 +2407,32 @@ void launch_batched(const In &in, const Out &out, const Mats &M, const Params &P
                     int n_inst, int n_tiles, const Queue &Q, int parity, int32_t *err, cudaStream_t s,
                     const mpf3d_tuning &T, uint8_t *tile_flags) {
     const int sms = sms_of_current_device();
-    batched_sweep_kernel<<<sweep_blocks((uint32_t)n_tiles, 8, sms), dim3(32, 8, 1), 0, s>>>(
-        in, out, P0, inst, n_inst, Q, parity, tile_flags, (uint32_t)n_tiles);
+    launch_early(batched_sweep_kernel, sweep_blocks((uint32_t)n_tiles, 8, sms), dim3(32, 8), s, in, out, P0, inst,
+                 n_inst, Q, parity, tile_flags, (uint32_t)n_tiles);
     // one stream: the side-by-side launch of the compact step measured no
     // gain here; the work-list grids come from T (the sweep's 32 x 8 x 4
     // tiles are fixed by the instance table)
     const int g_iface = sms * T.iface_blocks_per_sm, g_general = sms * T.general_blocks_per_sm;
+    const dim3 b_iface(T.iface_threads), b_general(T.general_threads);
+    const bool sym = P0.sym_normals;
     if (P0.cells < PAIR_CELLS) {  // as the single domain's step
-        if (P0.sym_normals)
-            batched_octet_kernel<S, AMAX, 4><<<sms * 8, 128, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity, err);
-        else batched_octet_kernel<S, AMAX, 8><<<sms * 8, 128, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity, err);
+        launch_early(sym ? batched_octet_kernel<S, AMAX, 4> : batched_octet_kernel<S, AMAX, 8>, sms * 8, dim3(128), s,
+                     in, out, M, P0, inst, n_inst, Q, parity, err);
         return;
     }
     if (!P0.use_aniso) {
-        batched_isotropic_kernel<S, AMAX>
-            <<<g_general, T.general_threads, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity, err);
+        launch_early(batched_isotropic_kernel<S, AMAX>, g_general, b_general, s, in, out, M, P0, inst, n_inst, Q,
+                     parity, err);
         return;
     }
-#define BATCHED(NT)                                                                                                   \
-    do {                                                                                                              \
-        if (Q.split)                                                                                                  \
-            batched_pair_kernel<NT><<<g_iface, T.iface_threads, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity);     \
-        batched_trio_kernel<S, NT><<<g_iface, T.iface_threads, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity);      \
-        batched_general_kernel<S><<<g_general, T.general_threads, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity);   \
-        batched_rest_kernel<S, AMAX, NT><<<sms * 8, 128, 0, s>>>(in, out, M, P0, inst, n_inst, Q, parity, err);       \
-    } while (0)
-    if (P0.sym_normals) BATCHED(4);
-    else BATCHED(8);
-#undef BATCHED
+    if (Q.split)
+        launch_early(sym ? batched_pair_kernel<4> : batched_pair_kernel<8>, g_iface, b_iface, s, in, out, M, P0, inst,
+                     n_inst, Q, parity);
+    launch_early(sym ? batched_trio_kernel<S, 4> : batched_trio_kernel<S, 8>, g_iface, b_iface, s, in, out, M, P0,
+                 inst, n_inst, Q, parity);
+    launch_early(batched_general_kernel<S>, g_general, b_general, s, in, out, M, P0, inst, n_inst, Q, parity);
+    launch_early(sym ? batched_rest_kernel<S, AMAX, 4> : batched_rest_kernel<S, AMAX, 8>, sms * 8, dim3(128), s, in,
+                 out, M, P0, inst, n_inst, Q, parity, err);
 }
 
 }  // namespace

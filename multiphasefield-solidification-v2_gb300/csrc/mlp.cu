@@ -1,19 +1,15 @@
-// mlp.cu -- BF16 tensor-core kernels of the orientation surrogate: a
-// strided GEMM with fused bias/activation epilogue, the activation
-// derivative, column sums, the MSE loss gradient and a fused Adam update.
+// mlp.cu -- BF16 tensor-core GEMMs with a fused bias/activation epilogue, the
+// activation derivative, column sums, the MSE loss gradient and a fused Adam
+// update.
 //
 // No reference counterpart: the reference has no learned component.  The
-// network maps (2 quaternions, undercooling, anisotropy strength) to (growth
-// velocity ratio, grain-boundary inclination) for the batched bicrystal
-// engine; it is small (134,914 parameters), so one generic GEMM kernel with
-// arbitrary operand strides serves the forward pass (X W^T), the input
-// gradient (dZ W) and the weight gradient (dZ^T X) alike.
-//
-// Two GEMM kernels: K-major operands (the forward pass X W^T, K <= 256,
-// N <= 256) run on the fifth-generation tensor cores (tcgen05.mma with the
-// accumulator in tensor memory); transposed operands (the gradients) use
-// mma.sync.m16n8k16 (BF16 in, FP32 accumulate) from shared memory tiles:
-// 64 x 64 output tile per CTA, 4 warps of 32 x 32, k step 32.
+// surrogate's network (mpf3d/surrogate.py) runs its layers and their gradients in
+// mlp_net.cu; the loss and Adam kernels here complete its training step, and the
+// GEMMs are entry points of the library: K-major operands (K <= 256, N <= 256) and
+// gathered transposed ones on the fifth-generation tensor cores (tcgen05.mma with
+// the accumulator in tensor memory), and mma.sync.m16n8k16 (BF16 in, FP32
+// accumulate) from shared memory tiles for comparison: 64 x 64 output tile per
+// CTA, 4 warps of 32 x 32, k step 32.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
