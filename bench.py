@@ -219,9 +219,9 @@ def quiet_cells(solver, step_index):
 
 
 def committed_traffic():
-    """DRAM bytes per step of the three step kernels over the bench's timed
+    """DRAM bytes per step of the step kernels over the bench's timed
     steps 1-20, from the committed ncu summary (a 128 x 128 x 256 crop with the
-    same grain density, one kernel per capture, scaled 4x to 256^3 by area)."""
+    same grain density, scaled 4x to 256^3 by area)."""
     path = os.path.join(ROOT, "profiles", "compact_step_dram_crop128x128x256_steps1-20.md")
     try:
         for line in open(path):
@@ -304,7 +304,7 @@ def config_dict(args):
     nx, ny, nz = GRID
     return {"workload": f"3D random Voronoi {nx}x{ny}x{nz}, {N_GRAINS} grains in the bottom {SLAB} z-layers + "
                         f"liquid (N={N_GRAINS + 1}), tanh front, anisotropy+torque on, uniform cooling "
-                        "(config_3d.yaml), FP32 compact three-kernel step",
+                        "(config_3d.yaml), FP32 compact step",
             "grid": list(GRID), "phases": N_GRAINS + 1, "slots": args.slots, "steps": args.steps,
             "l2": "inputs larger than L2, no flush: the two state buffers' head arrays alone are "
                   "2 x 67 MB (> 129 MB L2), plus the stored records; each step reads the previous "
