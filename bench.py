@@ -296,7 +296,7 @@ def run_reference(args, rank):
 
 def launches_per_step(cells):
     """Kernels of a compact step with anisotropy: sweep and octet_kernel; sweep,
-    pair, trio, general and rest kernels from 2^19 cells."""
+    pair, trio, general and rest kernels on large domains (every workload here)."""
     return 5 if cells >= 1 << 19 else 2
 
 

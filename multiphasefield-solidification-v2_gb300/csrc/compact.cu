@@ -2156,12 +2156,20 @@ uint32_t sweep_blocks(uint32_t chunks, int rows, int sms) {
     return (chunks + n - 1u) / n;
 }
 
-// Cells from which a step's lists go to pair_kernel, trio_kernel and
-// general_kernel, and what they leave to rest_kernel; on smaller domains the
-// octets take everything.  us per step by octets / by kind, with one grain per
-// 1000 surface cells: 64 x 64 x 64 31 / 46, 96 x 96 x 64 47 / 49, 128^3 89 / 59;
-// 150 x 117 x 90 isotropic 86 / 31.
-constexpr int64_t PAIR_CELLS = 1 << 19;
+// Whether a step's lists go to the kernels by kind of cell (isotropic_kernel, or
+// pair_kernel, trio_kernel, general_kernel and rest_kernel) or all to the octets.
+// What decides is the number of listed cells, which the host does not know: for
+// a front along z it follows the plane, for a batch of bicrystals, most of whose
+// cells are listed, the cells.  us for 10 steps with dense output, octets / by
+// kind: 64 x 64 x 64 500 / 528, 70 x 90 x 77 (job) 1336 / 1238, 100 x 100 x 50 818 /
+// 607, 300 x 60 x 28 1088 / 673; isotropic, one kernel either way, 45 x 45 x 90 361 /
+// 344, 64 x 64 x 64 425 / 356, 100 x 100 x 50 673 / 430.  Batches of 32 x 32 x 64, 2 of
+// them 258 / 342, 6 of them 532 / 406; 4 isotropic ones 335 / 207.
+constexpr int64_t KIND_CELLS = 1 << 19, KIND_PLANE = 5120, KIND_PLANE_ISOTROPIC = 2000, KIND_CELLS_BATCH = 1 << 18;
+bool by_kind(const Params &P) {
+    return P.cells >= KIND_CELLS || (int64_t)P.nx * P.ny >= (P.use_aniso ? KIND_PLANE : KIND_PLANE_ISOTROPIC);
+}
+bool by_kind_batch(const Params &P) { return P.cells >= KIND_CELLS_BATCH || !P.use_aniso; }
 
 // general(stream) and interface(stream) launch the work-list kernels of a step;
 // interface's go to the caller stream's side stream, forked from s after the
@@ -2255,7 +2263,7 @@ void launch_step(const In &in, const Out &out, const Mats &M, const Params &P, c
     else if (T.sweep_zb == 8) SWEEP_LAUNCH(8);
     else SWEEP_LAUNCH(4);
 #undef SWEEP_LAUNCH
-    if (P.cells < PAIR_CELLS) {  // 8 blocks of 128 threads are resident per SM
+    if (!by_kind(P)) {  // 8 blocks of 128 threads are resident per SM
         launch_early(P.sym_normals ? octet_kernel<S, AMAX, 4> : octet_kernel<S, AMAX, 8>, sms * 8, dim3(128), s, in,
                      out, M, P, Q, parity, err);
         return;
@@ -2415,7 +2423,7 @@ void launch_batched(const In &in, const Out &out, const Mats &M, const Params &P
     const int g_iface = sms * T.iface_blocks_per_sm, g_general = sms * T.general_blocks_per_sm;
     const dim3 b_iface(T.iface_threads), b_general(T.general_threads);
     const bool sym = P0.sym_normals;
-    if (P0.cells < PAIR_CELLS) {  // as the single domain's step
+    if (!by_kind_batch(P0)) {
         launch_early(sym ? batched_octet_kernel<S, AMAX, 4> : batched_octet_kernel<S, AMAX, 8>, sms * 8, dim3(128), s,
                      in, out, M, P0, inst, n_inst, Q, parity, err);
         return;
