@@ -1167,7 +1167,9 @@ __device__ __forceinline__ void advance_clock(const Params &P) {
 // gridDim.x-th chunk, at most SWEEP_TILES tiles (distant ones: the tiles that are
 // not quiet lie together).  A lane per tile reads its flags (quiet), then the warps
 // share the others, one per warp and round; visit fills the warp's sink, flag_of
-// is a tile's place in fout, domain_of a chunk's instance.  A warp of its own for each of the 79 % quiet tiles of
+// is a tile's place in fout, domain_of its instance, or -1 for the rows of a chunk
+// beyond the domain's last: they are no tiles, are not listed, and have no flag (the
+// place that flag_of computes for one belongs to another tile).  A warp of its own for each of the 79 % quiet tiles of
 // a 256^3 step with 64 grains spent the time on starting blocks; us per step with a
 // block per chunk / with up to 128 tiles per block: 256^3 41 / 23, 512 x 512 x 256
 // 155 / 63 (64 tiles: 69, 32: 78), 24 bicrystals 92 / 79.  With consecutive chunks
@@ -1186,8 +1188,8 @@ __device__ __forceinline__ void sweep_tiles(const Queue &Q, uint32_t cells, int 
     __syncthreads();
     if (32u * threadIdx.y < SWEEP_TILES) {
         const uint32_t chunk = blockIdx.x + tlin / rows * gridDim.x, row = tlin % rows;
-        const bool in = chunk < chunks;
-        const int of = in ? domain_of(chunk) : 0;
+        const int of = chunk < chunks ? domain_of(chunk, row) : -1;
+        const bool in = of >= 0;
         const bool skip = in && quiet(of, chunk, row);
         if (skip && fout) fout[flag_of(chunk, row)] = 1;
         const unsigned mask = __ballot_sync(0xffffffffu, in && !skip);
@@ -1261,14 +1263,15 @@ __global__ void __launch_bounds__(512, 3) sweep_kernel(In in, Out out, Params P,
     };
     auto at = [&](int a, int b, int c) { return ((uint32_t)c * (uint32_t)P.ny + (uint32_t)b) * ntx + (uint32_t)a; };
     sweep_tiles<ZB>(
-        Q, P.cells32, parity, chunks, fout, [](uint32_t) { return 0; },
+        Q, P.cells32, parity, chunks, fout,
+        [&](uint32_t chunk, uint32_t row) { return tile_of(chunk, row).m < P.ny ? 0 : -1; },
         [&](uint32_t chunk, uint32_t row) {
             const Tile t = tile_of(chunk, row);
             return at(t.tx, t.m, t.kb);
         },
         [&](int, uint32_t chunk, uint32_t row) {
             const auto [tx, m, kb] = tile_of(chunk, row);
-            if (!T.flags || m >= P.ny) return false;
+            if (!T.flags) return false;
             // the 7 flags are loaded together (no short-circuit chain of loads)
             const uint32_t f0 = fin[at(tx, m, kb)];
             const uint32_t f1 = fin[at(tx + 1 < T.ntx ? tx + 1 : 0, m, kb)];
@@ -1283,7 +1286,7 @@ __global__ void __launch_bounds__(512, 3) sweep_kernel(In in, Out out, Params P,
             const Tile t = tile_of(chunk, row);
             const uint32_t plane = (uint32_t)P.nx * (uint32_t)P.ny;
             const int l = t.tx * 32 + (int)threadIdx.x;
-            sink.add(l < P.nx && t.m < P.ny ? sweep_column<ZB>(in, out, P, Q.split, l, t.m, t.kb * ZB) : 0u,
+            sink.add(l < P.nx ? sweep_column<ZB>(in, out, P, Q.split, l, t.m, t.kb * ZB) : 0u,
                      P.base + (uint32_t)(t.kb * ZB) * plane + (uint32_t)t.m * (uint32_t)P.nx + (uint32_t)l, plane);
         });
 }
@@ -1815,14 +1818,14 @@ __global__ void __launch_bounds__(256, 8) batched_sweep_kernel(In in, Out out, P
     uint8_t *fout = flags ? flags + (size_t)parity * 8 * n_tiles : nullptr;
     sweep_tiles<SWEEP_ZB>(
         Q, P0.cells32, parity, n_tiles, fout,
-        [&](uint32_t tile) { return find_instance_by_tile(inst, n_inst, (int)tile); },
+        [&](uint32_t tile, uint32_t) { return find_instance_by_tile(inst, n_inst, (int)tile); },
         [](uint32_t tile, uint32_t row) { return tile * 8u + row; },
         [&](int i, uint32_t tile, uint32_t row) {
             if (!flags) return false;
             const mpf3d_instance &I = inst[i];
             const WarpTile t(I, tile, row);
             const int bx = t.bx, m = t.m, kb = t.kb;
-            if (m >= I.ny) return true;  // a row past the instance's top
+            if (m >= I.ny) return true;  // a row past the instance's top: its flag has a place of its own
             // the 7 flags are loaded together (no short-circuit chain of loads)
             const uint32_t f0 = fin[tile * 8u + row];
             const uint32_t f1 = fin[t.at(bx + 1 < t.tx ? bx + 1 : 0, m, kb)];
