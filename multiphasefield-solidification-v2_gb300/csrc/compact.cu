@@ -187,22 +187,26 @@ __device__ __forceinline__ float lap7(const Params &P, const float (&v)[7]) {
 }
 
 // a b c . x y z with the roundings fixed.  The solid-liquid terms are written
-// with explicit roundings throughout, so that every kernel that inlines them,
-// and both forms of the interface update, give the same bits.
+// with explicit roundings throughout, so that every kernel that inlines them, and
+// all forms of the interface update, give the same bits.  The order is part of the
+// results: the two faces of an axis are differenced first, then the axes added, with
+// products fused into the sums.  Other orders change the last bits of lap_sl, and with
+// them now and then which phases of a cell are clipped: with the six faces summed one
+// after the other, one of 24 bicrystals differed by 2.5e-3 in a fraction after 20 steps.
 __device__ __forceinline__ float dot3(float a, float b, float c, float x, float y, float z) {
     return fmaf(c, z, fmaf(a, x, __fmul_rn(b, y)));
 }
 
-// sqrtf and __fdividef as this file is compiled (-prec-sqrt=false), for normal
-// numbers: without the scaling of subnormal ones
+// sqrtf as this file is compiled (-prec-sqrt=false) and the reciprocal of
+// __fdividef, for normal numbers: without the scaling of subnormal ones
 __device__ __forceinline__ float root(float x) {
     float y;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float ratio(float a, float b) {
+__device__ __forceinline__ float recip(float x) {
     float y;
-    asm("div.approx.ftz.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
@@ -245,26 +249,37 @@ __device__ __forceinline__ PointTerms point_terms(const Params &P, const Grad &G
     t.a = P.mu_a * fmaf(P.delta_a, fmaf(P.tan_a0, Sn, C), 1.0f);
     const float e = P.eps0 * t.a;
     t.e2 = G.valid ? e * e : P.e2_flat;
-    t.coef = P.mu_da * fmaf(-P.tan_a0, ratio(t.cs, Sn), ratio(t.cs, C));
+    t.coef = P.mu_da * fmaf(t.cs, recip(C), -__fmul_rn(P.tan_a0, __fmul_rn(t.cs, recip(Sn))));
     return t;
 }
 // d cos / d(grad phi); 0 below the floor
 __device__ __forceinline__ float3 dcos(const Grad &G, const PointTerms &t) {
-    const float ud = __fmul_rn(dot3(G.g.x, G.g.y, G.g.z, t.nx, t.ny, t.nz), __fmul_rn(__fmul_rn(G.ig, G.ig), G.ig));
-    return make_float3(fmaf(-ud, G.g.x, __fmul_rn(t.nx, G.ig)), fmaf(-ud, G.g.y, __fmul_rn(t.ny, G.ig)),
-                       fmaf(-ud, G.g.z, __fmul_rn(t.nz, G.ig)));
+    const float ud = dot3(G.g.x, G.g.y, G.g.z, t.nx, t.ny, t.nz), ig3 = __fmul_rn(__fmul_rn(G.ig, G.ig), G.ig);
+    return make_float3(fmaf(t.nx, G.ig, -__fmul_rn(__fmul_rn(ud, G.g.x), ig3)),
+                       fmaf(t.ny, G.ig, -__fmul_rn(__fmul_rn(ud, G.g.y), ig3)),
+                       fmaf(t.nz, G.ig, -__fmul_rn(__fmul_rn(ud, G.g.z), ig3)));
 }
 
-// lap_sl and b_sl of one solid at a cell from its facet there and the sums
-// over the six neighbours: flux, of (eps^2 at the cell + there)(phi_L there -
-// at the cell), and div, of the neighbours' da/d(grad phi) components along
-// their own axis, + side minus - side (aniso_term1_solid_3d :149-204,
-// torque_A11_3d :386-441 with A13_divergence_3d :344-383, calc_b_from_cos
-// :33-55).  L: liquid at the 7 points; hxy, hxz, hyz: its mixed differences.
+// The flux through the + face of an axis less that through its - face: wp, wm are
+// eps^2 at the cell + at the neighbour, dp, dm phi_L there - at the cell.
+__device__ __forceinline__ float face_difference(float wp, float dp, float wm, float dm) {
+    return fmaf(wp, dp, __fmul_rn(wm, dm));
+}
+
+// lap_sl and b_sl of one solid at a cell from its facet there and, per axis, the
+// difference of the two faces' fluxes (flux) and of the neighbours' da/d(grad phi)
+// components along the axis, + side minus - side (div) (aniso_term1_solid_3d
+// :149-204, torque_A11_3d :386-441 with A13_divergence_3d :344-383,
+// calc_b_from_cos :33-55).  L: liquid at the 7 points; hxy, hxz, hyz: its mixed
+// differences.
+__device__ __forceinline__ float flux_sum(const Params &P, const float (&flux)[3]) {
+    const float h = P.inv_2dx * P.inv_dx;
+    return fmaf(flux[2], h, fmaf(flux[0], h, __fmul_rn(flux[1], h)));
+}
 __device__ __forceinline__ void center_terms(const Params &P, const Grad &G, const PointTerms &t, const float (&L)[7],
-                                             float hxy, float hxz, float hyz, float flux, float div, float &lap_sl,
-                                             float &b_sl) {
-    lap_sl = __fmul_rn(flux, P.inv_2dx * P.inv_dx);
+                                             float hxy, float hxz, float hyz, const float (&flux)[3],
+                                             const float (&div)[3], float &lap_sl, float &b_sl) {
+    lap_sl = flux_sum(P, flux);
     if (!G.valid) return;
     if (P.use_torque) {
         const float qq = 0.25f * P.inv_dx2;
@@ -279,21 +294,19 @@ __device__ __forceinline__ void center_terms(const Params &P, const Grad &G, con
         const float cxx = dot3(dc.x, dc.y, dc.z, pxx, pxy, pxz);
         const float cyy = dot3(dc.x, dc.y, dc.z, pxy, pyy, pyz);
         const float czz = dot3(dc.x, dc.y, dc.z, pxz, pyz, pzz);
-        const float dx = __fmul_rn(t.coef, dc.x), dy = __fmul_rn(t.coef, dc.y), dz = __fmul_rn(t.coef, dc.z);
-        // da/dx . da/d(grad phi) q + a div(da/d(grad phi)) q + a da/d(grad phi) . grad q
-        const float E1 = __fmul_rn(__fmul_rn(t.coef, G.q), dot3(cxx, cyy, czz, dx, dy, dz));
-        const float E2 = fmaf(__fmul_rn(t.a, G.q), __fmul_rn(div, P.half_over_dx), E1);
-        lap_sl = fmaf(P.eps0sq, fmaf(t.a, dot3(dx, dy, dz, qx, qy, qz), E2), lap_sl);
+        // per axis da/dx da/d(phi_x) q + a d(da/d(phi_x))/dx q + a da/d(phi_x) dq/dx
+        auto axis = [&](float c, float d_cos, float d, float dq) {
+            const float da = __fmul_rn(t.coef, d_cos), dd = __fmul_rn(d, P.half_over_dx);
+            const float e = fmaf(__fmul_rn(t.a, dd), G.q, __fmul_rn(__fmul_rn(__fmul_rn(t.coef, c), da), G.q));
+            return fmaf(__fmul_rn(t.a, da), dq, e);
+        };
+        const float Ex = axis(cxx, dc.x, div[0], qx), Ey = axis(cyy, dc.y, div[1], qy), Ez = axis(czz, dc.z, div[2], qz);
+        lap_sl = fmaf(P.eps0sq, __fadd_rn(__fadd_rn(Ex, Ey), Ez), lap_sl);
     }
     Facet f;
     f.valid = true;
     f.cabs = t.cabs; f.cs = t.cs; f.nx = t.nx; f.ny = t.ny; f.nz = t.nz; f.q = G.q;
     b_sl = calc_b(P, G.g, f);
-}
-
-// The sums over the six neighbours in the order of the octet's shuffles.
-__device__ __forceinline__ float arm_sum(const float (&f)[7]) {
-    return __fadd_rn(__fadd_rn(f[1], __fadd_rn(f[2], f[3])), __fadd_rn(__fadd_rn(f[4], f[5]), f[6]));
 }
 
 // Cell (l, m, k) and the steps to its neighbours in cell indices, modulo 2^32
@@ -342,9 +355,9 @@ struct Stencil {
         G[6] = (bottom) ? G[0] : make_float3((Lxpzm - Lxmzm) * g2, (Lypzm - Lymzm) * g2, (vL[0] - Lz2m) * g2);
         if (top) G[5].z = (vL[5] - vL[6]) * g2;
         if (bottom) G[6].z = (vL[5] - vL[6]) * g2;
-        hxy = (Lxpyp - Lxpym) - (Lxmyp - Lxmym);
-        hxz = (Lxpzp - Lxpzm) - (Lxmzp - Lxmzm);
-        hyz = (Lypzp - Lypzm) - (Lymzp - Lymzm);
+        hxy = Lxpyp - Lxpym - Lxmyp + Lxmym;
+        hxz = Lxpzp - Lxpzm - Lxmzp + Lxmzm;
+        hyz = Lypzp - Lypzm - Lymzp + Lymzm;
     }
 };
 
@@ -359,26 +372,32 @@ __device__ __forceinline__ void interface_terms(const Params &P, const Stencil &
 #pragma unroll
     for (int p = 1; p < 7; ++p)
         any = any || !(dot3(G[p].x, G[p].y, G[p].z, G[p].x, G[p].y, G[p].z) < P.g2_floor);
-    float flux[7], div[7];
+    float flux[3], div[3];
     if (!any) {  // flat liquid everywhere: eps^2 = (eps0 a(0))^2 at all 7 points, no torque
+        const float w = P.e2_flat + P.e2_flat;
 #pragma unroll
-        for (int p = 1; p < 7; ++p) flux[p] = __fmul_rn(P.e2_flat + P.e2_flat, L[p] - L[0]);
-        lap_sl = __fmul_rn(arm_sum(flux), P.inv_2dx * P.inv_dx);
+        for (int x = 0; x < 3; ++x) flux[x] = face_difference(w, L[1 + 2 * x] - L[0], w, L[2 + 2 * x] - L[0]);
+        lap_sl = flux_sum(P, flux);
         b_sl = P.b_flat;
         return;
     }
     const PointTerms t0 = point_terms<NT>(P, g0, un);
 #pragma unroll
-    for (int p = 1; p < 7; ++p) {
-        const Grad g(P, G[p]);
-        const PointTerms t = point_terms<NT>(P, g, un);
-        const float3 dc = dcos(g, t);
-        const float da = __fmul_rn(t.coef, p < 3 ? dc.x : (p < 5 ? dc.y : dc.z));
-        flux[p] = __fmul_rn(t0.e2 + t.e2, L[p] - L[0]);
-        div[p] = g.valid ? ((p & 1) ? da : -da) : 0.0f;
+    for (int x = 0; x < 3; ++x) {
+        float w[2], da[2];
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            const Grad g(P, G[1 + 2 * x + side]);
+            const PointTerms t = point_terms<NT>(P, g, un);
+            const float3 dc = dcos(g, t);
+            w[side] = t0.e2 + t.e2;
+            da[side] = g.valid ? __fmul_rn(t.coef, x == 0 ? dc.x : (x == 1 ? dc.y : dc.z)) : 0.0f;
+        }
+        flux[x] = face_difference(w[0], L[1 + 2 * x] - L[0], w[1], L[2 + 2 * x] - L[0]);
+        div[x] = __fsub_rn(da[0], da[1]);
     }
     b_sl = 1.0f;
-    center_terms(P, g0, t0, L, st.hxy, st.hxz, st.hyz, arm_sum(flux), arm_sum(div), lap_sl, b_sl);
+    center_terms(P, g0, t0, L, st.hxy, st.hxz, st.hyz, flux, div, lap_sl, b_sl);
 }
 
 // Three forms of the update of a queued cell give the same bits:
@@ -786,8 +805,9 @@ __device__ __forceinline__ bool octet_phases(const In &in, const Out &out, const
         const int q0 = O.axis == 0 ? 5 : (O.axis == 1 ? 1 : 3);
         const float Ap = from_lane(LA, q0), Am = from_lane(LA, q0 + 1), Bp = from_lane(LB, q0), Bm = from_lane(LB, q0 + 1);
         const float across = O.plus ? Ap - Am : Bp - Bm;
-        const float hxy = from_lane(beside, 1) - from_lane(beside, 2), hxz = from_lane(across, 1) - from_lane(across, 2);
-        const float hyz = from_lane(beside, 3) - from_lane(beside, 4);
+        const float hxy = from_lane(beside, 1) - from_lane(LA, 2) + from_lane(LB, 2);
+        const float hxz = from_lane(across, 1) - from_lane(LB, 5) + from_lane(LB, 6);
+        const float hyz = from_lane(beside, 3) - from_lane(LA, 4) + from_lane(LB, 4);
         const float3 g0 = make_float3((L[1] - L[2]) * P.inv_2dx, (L[3] - L[4]) * P.inv_2dx, (L[5] - L[6]) * P.inv_2dx);
         if (O.axis < 3) {
             const float u = along * P.inv_2dx, v = beside * P.inv_2dx, w = across * P.inv_2dx;
@@ -811,15 +831,12 @@ __device__ __forceinline__ bool octet_phases(const In &in, const Out &out, const
             if (t == ts) al = T.a;  // used from lane 7
             const float3 dc = dcos(G, T);
             const float e2_0 = from_lane(T.e2, 0);
-            const float da = __fmul_rn(T.coef, O.axis == 0 ? dc.x : (O.axis == 1 ? dc.y : dc.z));
-            // sums over the six arms (arm_sum's order)
-            float flux = O.axis < 3 ? __fmul_rn(e2_0 + T.e2, dL) : 0.0f;
-            float div = O.axis < 3 && G.valid ? (O.plus ? da : -da) : 0.0f;
-#pragma unroll
-            for (int o = 1; o < 8; o <<= 1) {
-                flux = __fadd_rn(flux, __shfl_xor_sync(ALL, flux, o));
-                div = __fadd_rn(div, __shfl_xor_sync(ALL, div, o));
-            }
+            const float da = G.valid ? __fmul_rn(T.coef, O.axis == 0 ? dc.x : (O.axis == 1 ? dc.y : dc.z)) : 0.0f;
+            // face_difference of each axis on its + lane, whose neighbour holds the - side
+            const float w = e2_0 + T.e2;
+            const float face = fmaf(w, dL, from_lane(__fmul_rn(w, dL), p + 1)), side = __fsub_rn(da, from_lane(da, p + 1));
+            const float flux[3] = {from_lane(face, 1), from_lane(face, 3), from_lane(face, 5)};
+            const float div[3] = {from_lane(side, 1), from_lane(side, 3), from_lane(side, 5)};
             float lv = 0.0f, b = any ? 1.0f : P.b_flat;
             if (p == 0 && solid) center_terms(P, G, T, L, hxy, hxz, hyz, flux, div, lv, b);
             __syncwarp();
