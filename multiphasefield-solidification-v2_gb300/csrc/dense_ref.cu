@@ -727,6 +727,7 @@ __global__ void __launch_bounds__(THREADS, PER_SM) update_kernel(Field<T> phi, T
     int l0, m0, k0;
     tile_origin<RX, RY, false>(P.nx, P.ny, P.nz, l0, m0, k0);
     const int k = k0 + lane;
+    bool listed = false;
     // zeros, one-phase cells, and each row's mask of the others
     for (int r = warp; r < ROWS; r += THREADS / 32) {
         const int l = l0 + r / RY, m = m0 + r % RY;
@@ -757,6 +758,7 @@ __global__ void __launch_bounds__(THREADS, PER_SM) update_kernel(Field<T> phi, T
             row_mask[0][r] = many;
             row_mask[1][r] = two;
         }
+        listed = listed || (many | two) != 0u;
         if (n >= 0) {
             T *out = phi_new + cell;
             for (int g = 0; g < N; ++g) out[(size_t)g * plane] = (T)0;
@@ -767,11 +769,9 @@ __global__ void __launch_bounds__(THREADS, PER_SM) update_kernel(Field<T> phi, T
             }
         }
     }
-    __syncthreads();
-    uint32_t any = 0;
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) any |= row_mask[0][r] | row_mask[1][r];
-    if (!any) return;
+    // one answer for the block: the crew below changes row_mask, which a late warp
+    // must not read to decide whether to stay
+    if (!__syncthreads_or(listed)) return;
     // the last warp evaluates the shared values, the others collect the cells
     constexpr int CREW = THREADS - 32;
     if (threadIdx.x >= CREW) {
