@@ -166,6 +166,10 @@ __device__ __forceinline__ uint32_t cidx(const Params &P, int l, int m, int k) {
     return P.base + ((uint32_t)k * (uint32_t)P.ny + (uint32_t)m) * (uint32_t)P.nx + (uint32_t)l;
 }
 
+// place of slot s of cell c in the idx and val arrays.  Slots beyond the second may lie
+// past 2^32 entries in states that the step accepts (2^31 cells).
+__device__ __forceinline__ size_t slot_at(uint32_t s, uint32_t cells, uint32_t c) { return (size_t)s * cells + c; }
+
 // liquid fraction of cell q; the head and the first value are loaded
 // together (the value is ignored where the head says it is not needed), so
 // the liquid stencil costs one round of loads rather than two
@@ -513,8 +517,8 @@ __device__ __forceinline__ bool trio_cell(const In &in, const Out &out, const Ma
         ic[p] = NONE;
         vd[p] = 0.0f;
         if (n > 2) {
-            ic[p] = (int)__ldg(in.idx + 2u * cells + pt[p]);
-            vd[p] = __ldg(in.val + 2u * cells + pt[p]);
+            ic[p] = (int)__ldg(in.idx + slot_at(2, cells, pt[p]));
+            vd[p] = __ldg(in.val + slot_at(2, cells, pt[p]));
         }
         fits = fits && n <= 3;
     }
@@ -640,8 +644,8 @@ __device__ __forceinline__ bool trio_cell(const In &in, const Out &out, const Ma
         const float v = normal ? o[t] * inv : o[t];
         if (t >= n || !(v > 0.0f) || (!normal && ids[t] == LIQ)) continue;
         if (stored == 0) first = ids[t];
-        else out.idx[(uint32_t)stored * cells + c] = (uint16_t)ids[t];
-        out.val[(uint32_t)stored * cells + c] = v;
+        else out.idx[slot_at(stored, cells, c)] = (uint16_t)ids[t];
+        out.val[slot_at(stored, cells, c)] = v;
         ++stored;
     }
     // one stored phase: its renormalised value is 1 and is left implicit
@@ -750,8 +754,8 @@ __device__ __forceinline__ bool octet_phases(const In &in, const Out &out, const
             ++pos;
             nid = NONE;
             if (pos + 1 < cnt) {
-                nid = (int)__ldg(in.idx + (uint32_t)(pos + 1) * cells + pt);
-                nval = __ldg(in.val + (uint32_t)(pos + 1) * cells + pt);
+                nid = (int)__ldg(in.idx + slot_at(pos + 1, cells, pt));
+                nval = __ldg(in.val + slot_at(pos + 1, cells, pt));
             }
         }
         const float v[7] = {from_lane(own, 0), from_lane(own, 1), from_lane(own, 2), from_lane(own, 3), from_lane(own, 4), from_lane(own, 5), from_lane(own, 6)};
@@ -925,8 +929,8 @@ __device__ __forceinline__ bool octet_phases(const In &in, const Out &out, const
         const int id = from_lane(ids[h], max(__ffs(mask) - 1, 0));
         if (stored == 0 && mask) id_first = id;
         if (writes && keep && at < S) {
-            if (at > 0) out.idx[(uint32_t)at * cells + c] = (uint16_t)ids[h];
-            out.val[(uint32_t)at * cells + c] = v;
+            if (at > 0) out.idx[slot_at(at, cells, c)] = (uint16_t)ids[h];
+            out.val[slot_at(at, cells, c)] = v;
         }
         stored += __popc(mask);
     }
@@ -938,8 +942,8 @@ __device__ __forceinline__ bool octet_phases(const In &in, const Out &out, const
             const int c0 = min(hcount(hw), S);
             out.head[c] = hw;
             for (int s = 0; s < c0; ++s) {
-                out.idx[(uint32_t)s * cells + c] = __ldg(in.idx + (uint32_t)s * cells + c);
-                out.val[(uint32_t)s * cells + c] = __ldg(in.val + (uint32_t)s * cells + c);
+                out.idx[slot_at(s, cells, c)] = __ldg(in.idx + slot_at(s, cells, c));
+                out.val[slot_at(s, cells, c)] = __ldg(in.val + slot_at(s, cells, c));
             }
         } else {
             if (!normal) out.val[c] = 1.0f;
