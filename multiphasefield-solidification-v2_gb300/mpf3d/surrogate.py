@@ -189,10 +189,17 @@ class Surrogate:
 
     def backward(self, dout) -> None:
         """Gradients of the loss w.r.t. all parameters into self.g, given the
-        FP32 gradient w.r.t. the outputs [M, 2]."""
+        FP32 gradient w.r.t. the outputs: [M, 2], or of the first rows only
+        (the others then take no part in the loss)."""
         t = self.torch
         x16, Z, Y = self._saved
-        M = dout.shape[0]
+        M = x16.shape[0]  # what the forward pass kept is laid out by its rows
+        if dout.shape[0] > M:
+            raise ValueError(f"gradient of {dout.shape[0]} rows for a forward pass of {M}")
+        if dout.shape[0] < M:
+            whole = t.zeros((M, OUT), dtype=t.float32, device=self.device)
+            whole[:dout.shape[0]] = dout
+            dout = whole
         dz = t.empty(M * (3 * HIDDEN + 8), dtype=t.int16, device=self.device)
         partial = t.empty(-(-M // 128) * 4 * 3 * HIDDEN, dtype=t.float32, device=self.device)
         rc = _lib.lib().mpf3d_mlp_backward(M, x16.data_ptr(), self.w16.data_ptr(), Z.data_ptr(), Y.data_ptr(),
