@@ -176,6 +176,8 @@ class Surrogate:
         backward pass needs."""
         t = self.torch
         M = x16.shape[0]
+        if x16.data_ptr() % 16:  # a view at an odd offset: the kernels read 16 bytes at a time
+            x16 = x16.clone()
         out = t.empty((M, OUT), dtype=t.float32, device=self.device)
         Z = t.empty((3, HIDDEN // 4, M, 4), dtype=t.float32, device=self.device) if keep else None
         Y = t.empty((3, M, HIDDEN), dtype=t.int16, device=self.device) if keep else None
@@ -196,7 +198,7 @@ class Surrogate:
         M = x16.shape[0]  # what the forward pass kept is laid out by its rows
         if dout.shape[0] > M:
             raise ValueError(f"gradient of {dout.shape[0]} rows for a forward pass of {M}")
-        if dout.shape[0] < M:
+        if dout.shape[0] < M or dout.data_ptr() % 8:
             whole = t.zeros((M, OUT), dtype=t.float32, device=self.device)
             whole[:dout.shape[0]] = dout
             dout = whole
