@@ -972,6 +972,164 @@ __device__ __forceinline__ void octet_cell(const In &in, const Out &out, const M
         octet_many<S, AMAX, NT>(in, out, M, P, err, O, active, l, m, k);
 }
 
+// ---------------------------------------------------------------------------
+// Any queued cell, one thread: the lists merged and the pair sums formed in arrays of
+// local memory, a phase at a time.  A cell takes several times as long as by an octet,
+// but 32 of them share a warp where octets have four: the better form where the cells
+// are many (see Lists::are_long, EVERYWHERE and MANY_LEFT).
+// FACETS: the anisotropic solid-liquid terms, for cells that have them.
+template <int S, int AMAX, bool FACETS, int NT>
+__device__ __forceinline__ void any_cell(const In &in, const Out &out, const Mats &M, const Params &P,
+                                         int32_t *__restrict__ err, int l, int m, int k) {
+    constexpr int NONE = 0x7fffffff;
+    const uint32_t cells = P.cells32;
+    const Offsets o(P, l, m, k);
+    const uint32_t c = o.c, pt[7] = {c, c + o.xp, c + o.xm, c + o.yp, c + o.ym, c + o.zp, c + o.zm};
+    int n = 0, ts = -1, ids[AMAX];
+    float vc[AMAX], lap[AMAX], vL[7], maxv = -1.0f;
+    float3 gs = make_float3(0.f, 0.f, 0.f);
+    bool ovf = false;
+    uint32_t hw[7];
+    int pos[7], next[7];
+#pragma unroll
+    for (int p = 0; p < 7; ++p) {
+        hw[p] = __ldg(in.head + pt[p]);
+        pos[p] = 0;
+        next[p] = hcount(hw[p]) > 0 ? hid0(hw[p]) : NONE;
+        vL[p] = 0.0f;
+    }
+    while (true) {
+        int id = next[0];
+#pragma unroll
+        for (int p = 1; p < 7; ++p) id = min(id, next[p]);
+        if (id == NONE) break;
+        float v[7];
+#pragma unroll
+        for (int p = 0; p < 7; ++p) {
+            v[p] = 0.0f;
+            if (next[p] != id) continue;
+            v[p] = pos[p] == 0 ? value0(in, hw[p], pt[p]) : __ldg(in.val + slot_at(pos[p], cells, pt[p]));
+            ++pos[p];
+            next[p] = pos[p] < min(hcount(hw[p]), S) ? (int)__ldg(in.idx + slot_at(pos[p], cells, pt[p])) : NONE;
+        }
+        if (n == AMAX) {
+            ovf = true;
+            break;
+        }
+        ids[n] = id;
+        vc[n] = v[0];
+        lap[n] = lap7(P, v);
+        if (id == LIQ) {
+#pragma unroll
+            for (int p = 0; p < 7; ++p) vL[p] = v[p];
+        } else if (v[0] > maxv) {
+            maxv = v[0];
+            ts = n;
+            gs = make_float3((v[1] - v[2]) * P.inv_2dx, (v[3] - v[4]) * P.inv_2dx, (v[5] - v[6]) * P.inv_2dx);
+        }
+        ++n;
+    }
+    if (ovf) {
+        // leave the cell as it was and report; the host re-runs the step with a
+        // wider template
+        atomicOr(err, MPF3D_DEV_SLOT_OVERFLOW);
+        out.head[c] = hw[0];
+        for (int t = 0; t < min(hcount(hw[0]), S); ++t) {
+            out.idx[slot_at(t, cells, c)] = __ldg(in.idx + slot_at(t, cells, c));
+            out.val[slot_at(t, cells, c)] = __ldg(in.val + slot_at(t, cells, c));
+        }
+        return;
+    }
+    // solid-liquid terms
+    const bool heavy = n > 1 && ids[0] == LIQ, facets = FACETS && heavy && P.use_aniso;
+    const float lap_iso = heavy ? P.eps0sq * lap[0] : 0.0f;  // isotropic branch of the switchable kernel (:729-731)
+    float lap_sl[AMAX], b_sl[AMAX], w_sl = P.w0;
+    if (facets) {
+        const Stencil st(in, P, o, vL);
+        lap_sl[0] = 0.0f;
+        b_sl[0] = 1.0f;
+#pragma unroll 1
+        for (int t = 1; t < n; ++t) {
+            const float *ug = M.n111 + (size_t)(P.n111_base + ids[t]) * 24;
+            float un[3 * NT], lv, b;
+#pragma unroll
+            for (int q = 0; q < 3 * NT; ++q) un[q] = __ldg(ug + q);
+            interface_terms<NT>(P, st, vL, un, lv, b);
+            lap_sl[t] = lv;
+            b_sl[t] = b;
+            if (t == ts) {
+                const float al = point_terms<NT>(P, Grad(P, gs), un).a;
+                w_sl = P.w0 * (al * al);
+            }
+        }
+    }
+    // pair sums (trio_cell)
+    const int N = P.N;
+    float W[AMAX], Ag[AMAX], outv[AMAX];
+#pragma unroll 1
+    for (int t = 0; t < n; ++t) {
+        const int i = ids[t];
+        float w = 0.0f, a = 0.0f;
+#pragma unroll 1
+        for (int q = 0; q < n; ++q) {
+            const float wik = ids[q] == LIQ && i != LIQ ? w_sl : __ldg(M.wij + i * N + ids[q]);
+            w = fmaf(wik, vc[q], w);
+            a = fmaf(__ldg(M.a2ij + i * N + ids[q]), lap[q], a);
+        }
+        W[t] = w;
+        Ag[t] = a;
+    }
+    const double Tmc = P.clock ? P.clock->tmc[P.parity] : P.Tmc;
+    const float dT = P.t_uniform ? P.dT_uniform : (float)(M.T0z[k] - Tmc);
+    const float inv_n = 1.0f / (float)(n > 0 ? n : 1);
+    float sum = 0.0f, low = 0.0f;
+#pragma unroll 1
+    for (int t = 0; t < n; ++t) {
+        const int i = ids[t];
+        float dpi = 0.0f;
+#pragma unroll 1
+        for (int q = 0; q < n; ++q) {
+            if (q == t) continue;
+            const int j = ids[q];
+            const bool sl = i != LIQ && j == LIQ, ls = i == LIQ && j != LIQ;
+            const float l1 = sl && facets ? lap_sl[t] : lap_iso, l2 = ls && facets ? lap_sl[q] : lap_iso;
+            const float T = sl ? 0.5f * l1 : (ls ? -0.5f * l2 : 0.5f * __fsub_rn(Ag[t], Ag[q]));
+            const float ppp = __fadd_rn(__fsub_rn(W[t], W[q]), T);
+            const float df = sl ? -P.Sf * dT : (ls ? P.Sf * dT : 0.0f);
+            const float tf = __fmul_rn(__fmul_rn(FORCE_PREF, sqrtf(fmaxf(__fmul_rn(vc[t], vc[q]), 0.0f))), df);
+            float me = __ldg(M.mij + i * N + j);
+            if (facets) me = sl ? me * b_sl[t] : (ls ? me * b_sl[q] : me);
+            dpi = __fsub_rn(dpi, __fmul_rn(__fmul_rn(__fmul_rn(2.0f, me), inv_n), __fsub_rn(ppp, tf)));
+        }
+        outv[t] = fminf(fmaxf(fmaf(P.dt, dpi, vc[t]), 0.0f), 1.0f);
+        // compensated (TwoSum) float accumulation (:663-680)
+        const float s2 = sum + outv[t], bb = s2 - sum;
+        low += (sum - (s2 - bb)) + (outv[t] - bb);
+        sum = s2;
+    }
+    // stored list: the phases that stay positive, ascending; all clipped to
+    // ~0: the liquid takes the cell (:679-680)
+    const bool normal = sum + low > 1e-20f;
+    float inv = 1.0f / sum;
+    inv = fmaf(-__fmul_rn(inv, inv), low, inv);
+    int stored = normal ? 0 : 1, first = LIQ;
+    if (!normal) out.val[c] = 1.0f;
+#pragma unroll 1
+    for (int t = 0; t < n; ++t) {
+        const float v = normal ? outv[t] * inv : outv[t];
+        if (!(v > 0.0f) || (!normal && ids[t] == LIQ)) continue;
+        if (stored < S) {
+            if (stored == 0) first = ids[t];
+            else out.idx[slot_at(stored, cells, c)] = (uint16_t)ids[t];
+            out.val[slot_at(stored, cells, c)] = v;
+        }
+        ++stored;
+    }
+    // one stored phase: its renormalised value is 1 and is left implicit
+    out.head[c] = mkhead(first, min(stored, S), false);
+    if (stored > S) atomicOr(err, MPF3D_DEV_SLOT_OVERFLOW);
+}
+
 // Kernel 1 of a step: every cell.  Uniform neighbourhoods (the cell and its
 // 6 neighbours hold one and the same phase: active list of one phase, empty
 // pair sums, renormalised fraction exactly 1) are written directly; every
@@ -1471,6 +1629,13 @@ __global__ void __launch_bounds__(512, 3) sweep_kernel_tma(const __grid_constant
     sink.flush(Q, P.cells32, s_base);
 }
 
+// Lists so long that a thread per cell gets through them sooner than eight lanes: us a
+// step by octets / by threads, 64 x 64 x 64 with two grains and 61 k cells listed 29.5 /
+// 23.2, with 8 grains and 70 k 37.9 / 42.4, 113 k 47.3 / 40.8; 32 x 32 x 64 isotropic,
+// 44 k 25.8 / 25.5, 58 k 31.5 / 27.0, with 20 k 16.2 / 19.5.  Cells with several solids, the
+// costly ones, weigh more: 48 x 40 x 56 with 54 k of them 134 / 66.
+constexpr uint32_t LONG_LISTS = 49152, LONG_SEVERAL = 16384;
+
 // The work lists: 0 at items[0..), 1 at items[cells-1..] downwards, 2 at
 // items[cells..).
 struct Lists {
@@ -1480,6 +1645,9 @@ struct Lists {
         n[1] = *(volatile uint32_t *)(Q.count + 2 * parity + 1);
         n[2] = Q.split ? *(volatile uint32_t *)(Q.count + 4 + parity) : 0u;
     }
+    __device__ __forceinline__ bool are_long() const {
+        return n[2] > LONG_SEVERAL || n[0] + n[1] + n[2] > LONG_LISTS;
+    }
     // index in items of entry i of the lists one after the other
     __device__ __forceinline__ uint32_t item(uint32_t i, uint32_t cells) const {
         if (i < n[0]) return i;
@@ -1488,11 +1656,21 @@ struct Lists {
     }
 };
 
-// calls cell(c, active) for the cells of all lists, four per warp and call
-template <class Cell>
-__device__ __forceinline__ void for_octets(const Queue &Q, uint32_t cells, int parity, Cell &&cell) {
+// resident blocks of 128 threads per SM of octet_kernel: registers for any_cell, and
+// still a wave for 12 k cells
+constexpr int OCTET_BLOCKS = 5;
+
+// calls cell(c, active) for the cells of all lists, four per warp and call, or where
+// they are long each(c, of list 0?), one per thread
+template <class Cell, class Each>
+__device__ __forceinline__ void for_octets(const Queue &Q, uint32_t cells, int parity, Cell &&cell, Each &&each) {
     const Lists L(Q, parity);
     const uint32_t n = L.n[0] + L.n[1] + L.n[2], oct = (threadIdx.x & 31u) >> 3;
+    if (L.are_long()) {
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+            each(Q.items[L.item(i, cells)], i < L.n[0]);
+        return;
+    }
     const uint32_t warps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     for (uint32_t w = warp; w * 4u < n; w += warps) {
         const uint32_t i = w * 4u + oct;
@@ -1506,10 +1684,13 @@ __device__ __forceinline__ void for_octets(const Queue &Q, uint32_t cells, int p
 // each, one after the other.  For the same reason a block takes runs of RUN
 // items from distant parts of the range; PER: items that make another block
 // worth starting.
-constexpr uint32_t LEFT_CELLS = 1024;
+// With EACH, a block that is left with more than MANY_LEFT of them, and more than half of
+// its items, does them by each(item), one per thread (64 x 64 x 64 isotropic, 140 k cells
+// with 9 phases: 379 us a step by octets, 136 so).
+constexpr uint32_t LEFT_CELLS = 1024, MANY_LEFT = 96;
 
-template <uint32_t RUN, uint32_t PER, class Get, class Take, class Rest>
-__device__ __forceinline__ void for_items(uint32_t n, Get &&get, Take &&take, Rest &&rest) {
+template <uint32_t RUN, uint32_t PER, bool EACH, class Get, class Take, class Rest, class Each>
+__device__ __forceinline__ void for_items(uint32_t n, Get &&get, Take &&take, Rest &&rest, Each &&each) {
     __shared__ uint32_t left[LEFT_CELLS], n_left;
     const uint32_t blocks = min(gridDim.x, (n + PER - 1u) / PER);
     if (blockIdx.x >= blocks) return;
@@ -1518,6 +1699,7 @@ __device__ __forceinline__ void for_items(uint32_t n, Get &&get, Take &&take, Re
     if (threadIdx.x == 0) n_left = 0;
     __syncthreads();
     for (uint32_t at0 = 0; at0 < n;) {
+        const uint32_t first = at0;
         for (uint32_t pass = 0; pass < passes && at0 < n; ++pass, at0 += step) {
             const uint32_t i = at0 + (threadIdx.x / RUN * blocks + blockIdx.x) * RUN + threadIdx.x % RUN;
             if (i >= n) continue;
@@ -1526,8 +1708,12 @@ __device__ __forceinline__ void for_items(uint32_t n, Get &&get, Take &&take, Re
         }
         __syncthreads();
         const uint32_t m = n_left;
-        for (uint32_t w = warp; w * 4u < m; w += blockDim.x >> 5)
-            rest(left[min(w * 4u + oct, m - 1u)], w * 4u + oct < m);
+        if (EACH && m > MANY_LEFT && 2u * m > (min(at0, n) - first) / blocks) {
+            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) each(left[i]);
+        } else {
+            for (uint32_t w = warp; w * 4u < m; w += blockDim.x >> 5)
+                rest(left[min(w * 4u + oct, m - 1u)], w * 4u + oct < m);
+        }
         __syncthreads();
         if (threadIdx.x == 0) n_left = 0;
         __syncthreads();
@@ -1553,13 +1739,17 @@ struct Place {
 // Kernel 2 of a step on small domains: eight lanes per cell.  NT: normals per
 // grain (4 or 8, from P.sym_normals).
 template <int S, int AMAX, int NT>
-__global__ void __launch_bounds__(128, 8) octet_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity,
+__global__ void __launch_bounds__(128, OCTET_BLOCKS) octet_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity,
                                                        int32_t *__restrict__ err) {
     wait_for_previous();
     const OctetLane O;
     for_octets(Q, P.cells32, parity, [&](uint32_t c, bool active) {
         const Place at(c, P.nx, P.ny);
         octet_cell<S, AMAX, NT>(in, out, M, P, err, O, active, at.l, at.m, at.k);
+    }, [&](uint32_t c, bool general) {
+        const Place at(c, P.nx, P.ny);
+        if (!general || !trio_cell<S, false, 4>(in, out, M, P, at.l, at.m, at.k))
+            any_cell<S, AMAX, true, NT>(in, out, M, P, err, at.l, at.m, at.k);
     });
 }
 
@@ -1574,11 +1764,26 @@ __global__ void __launch_bounds__(128, 5) pair_kernel(In in, Out out, Mats M, Pa
     }
 }
 
-// list 2: multi-solid interface cells
-template <int S, int NT>
-__global__ void __launch_bounds__(128, 4) trio_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity) {
+// list 2: multi-solid interface cells.  Where there are far more of them than one-solid
+// cells, a melt solidifies everywhere at once and its cells hold a phase of most grains:
+// they go to any_cell instead of trio_cell in vain and then the octets (160 x 160 x 32 with
+// 229 k of them 512 / 241 us a step, 128 x 128 x 64 with 500 grains and 205 k 243 / 205; with
+// 50 k of them 75 / 85).  With a front, list 2 is at most 1.5 times as long as list 1.
+constexpr uint32_t EVERYWHERE = 60000;
+template <int S, int AMAX, int NT>
+__global__ void __launch_bounds__(128, 4) trio_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity,
+                                                      int32_t *__restrict__ err) {
     wait_for_previous();
-    const uint32_t n = *(volatile uint32_t *)(Q.count + (Q.split ? 4 + parity : 2 * parity + 1));
+    // loads that are in flight together
+    const uint32_t one = __ldcg(Q.count + 2 * parity + 1), several = __ldcg(Q.count + (Q.split ? 4 : 2) + parity);
+    const uint32_t n = Q.split ? several : one;
+    if (Q.split && several > EVERYWHERE && several / 8u > one) {
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+            const Place at(Q.items[P.cells32 + i], P.nx, P.ny);
+            any_cell<S, AMAX, true, NT>(in, out, M, P, err, at.l, at.m, at.k);
+        }
+        return;
+    }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t &item = Q.items[Q.split ? P.cells32 + i : P.cells32 - 1u - i];
         const uint32_t c = item;
@@ -1607,14 +1812,15 @@ __global__ void __launch_bounds__(128, 8)
     const OctetLane O;
     Lists L(Q, parity);
     if (Q.split) L.n[1] = 0;
-    for_items<8, 32>(
+    for_items<8, 32, false>(
         L.n[0] + L.n[1] + L.n[2], [&](uint32_t i) { return Q.items[L.item(i, P.cells32)]; },
         [](uint32_t c) { return (c & LEFT) == 0u; },
         [&](uint32_t marked, bool active) {
             const uint32_t c = marked & ~LEFT;
             const Place at(c, P.nx, P.ny);
             octet_cell<S, AMAX, NT>(in, out, M, P, err, O, active, at.l, at.m, at.k);
-        });
+        },
+        [](uint32_t) {});
 }
 
 // list 0 of the isotropic model, which has no other: what trio_cell leaves is
@@ -1624,7 +1830,7 @@ __global__ void __launch_bounds__(256, 3)
     isotropic_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity, int32_t *__restrict__ err) {
     wait_for_previous();
     const OctetLane O;
-    for_items<32, 256>(
+    for_items<32, 256, true>(
         *(volatile uint32_t *)(Q.count + 2 * parity), [&](uint32_t i) { return Q.items[i]; },
         [&](uint32_t c) {
             const Place at(c, P.nx, P.ny);
@@ -1633,6 +1839,10 @@ __global__ void __launch_bounds__(256, 3)
         [&](uint32_t c, bool active) {
             const Place at(c, P.nx, P.ny);
             octet_cell<S, AMAX, 4>(in, out, M, P, err, O, active, at.l, at.m, at.k);
+        },
+        [&](uint32_t c) {
+            const Place at(c, P.nx, P.ny);
+            any_cell<S, AMAX, false, 4>(in, out, M, P, err, at.l, at.m, at.k);
         });
 }
 
@@ -1871,7 +2081,7 @@ __global__ void __launch_bounds__(256, 8) batched_sweep_kernel(In in, Out out, P
 // The work-list kernels of a batch: as the single domain's, on the instance of
 // each cell.
 template <int S, int AMAX, int NT>
-__global__ void __launch_bounds__(128, 8) batched_octet_kernel(In in, Out out, Mats M, Params P0,
+__global__ void __launch_bounds__(128, OCTET_BLOCKS) batched_octet_kernel(In in, Out out, Mats M, Params P0,
                                                                const mpf3d_instance *__restrict__ inst, int n_inst,
                                                                Queue Q, int parity, int32_t *__restrict__ err) {
     wait_for_previous();
@@ -1880,6 +2090,12 @@ __global__ void __launch_bounds__(128, 8) batched_octet_kernel(In in, Out out, M
         const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
         const Place at(c - I.offset, I.nx, I.ny);
         octet_cell<S, AMAX, NT>(in, out, M, instance_params(P0, I), err, O, active, at.l, at.m, at.k);
+    }, [&](uint32_t c, bool general) {
+        const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
+        const Place at(c - I.offset, I.nx, I.ny);
+        const Params P = instance_params(P0, I);
+        if (!general || !trio_cell<S, false, 4>(in, out, M, P, at.l, at.m, at.k))
+            any_cell<S, AMAX, true, NT>(in, out, M, P, err, at.l, at.m, at.k);
     });
 }
 
@@ -1900,7 +2116,7 @@ __global__ void __launch_bounds__(128, 5) batched_pair_kernel(In in, Out out, Ma
 // list 2: multi-solid interface cells
 template <int S, int NT>
 __global__ void __launch_bounds__(128, 4) batched_trio_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity) {
-    wait_for_previous();
+    wait_for_previous();  // two grains and the liquid: trio_cell takes every cell of a batch's bicrystals
     const uint32_t n = *(volatile uint32_t *)(Q.count + (Q.split ? 4 + parity : 2 * parity + 1));
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t &item = Q.items[Q.split ? P0.cells32 + i : P0.cells32 - 1u - i];
@@ -1932,7 +2148,7 @@ __global__ void __launch_bounds__(128, 8)
     const OctetLane O;
     Lists L(Q, parity);
     if (Q.split) L.n[1] = 0;
-    for_items<8, 32>(
+    for_items<8, 32, false>(
         L.n[0] + L.n[1] + L.n[2], [&](uint32_t i) { return Q.items[L.item(i, P0.cells32)]; },
         [](uint32_t c) { return (c & LEFT) == 0u; },
         [&](uint32_t marked, bool active) {
@@ -1940,7 +2156,8 @@ __global__ void __launch_bounds__(128, 8)
             const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
             const Place at(c - I.offset, I.nx, I.ny);
             octet_cell<S, AMAX, NT>(in, out, M, instance_params(P0, I), err, O, active, at.l, at.m, at.k);
-        });
+        },
+        [](uint32_t) {});
 }
 
 // list 0 of the isotropic model, which has no other: what trio_cell leaves is
@@ -1950,7 +2167,7 @@ __global__ void __launch_bounds__(256, 3)
     batched_isotropic_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity, int32_t *__restrict__ err) {
     wait_for_previous();
     const OctetLane O;
-    for_items<32, 256>(
+    for_items<32, 256, true>(
         *(volatile uint32_t *)(Q.count + 2 * parity), [&](uint32_t i) { return Q.items[i]; },
         [&](uint32_t c) {
             const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
@@ -1961,6 +2178,11 @@ __global__ void __launch_bounds__(256, 3)
             const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
             const Place at(c - I.offset, I.nx, I.ny);
             octet_cell<S, AMAX, 4>(in, out, M, instance_params(P0, I), err, O, active, at.l, at.m, at.k);
+        },
+        [&](uint32_t c) {
+            const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
+            const Place at(c - I.offset, I.nx, I.ny);
+            any_cell<S, AMAX, false, 4>(in, out, M, instance_params(P0, I), err, at.l, at.m, at.k);
         });
 }
 
@@ -2181,17 +2403,20 @@ uint32_t sweep_blocks(uint32_t chunks, int rows, int sms) {
 }
 
 // Whether a step's lists go to the kernels by kind of cell (isotropic_kernel, or
-// pair_kernel, trio_kernel, general_kernel and rest_kernel) or all to the octets.
-// What decides is the number of listed cells, which the host does not know: for
-// a front along z it follows the plane, for a batch of bicrystals, most of whose
-// cells are listed, the cells.  us for 10 steps with dense output, octets / by
-// kind: 64 x 64 x 64 500 / 528, 70 x 90 x 77 (job) 1336 / 1238, 100 x 100 x 50 818 /
-// 607, 300 x 60 x 28 1088 / 673; isotropic, one kernel either way, 45 x 45 x 90 361 /
-// 344, 64 x 64 x 64 425 / 356, 100 x 100 x 50 673 / 430.  Batches of 32 x 32 x 64, 2 of
-// them 258 / 342, 6 of them 532 / 406; 4 isotropic ones 335 / 207.
-constexpr int64_t KIND_CELLS = 1 << 19, KIND_PLANE = 5120, KIND_PLANE_ISOTROPIC = 2000, KIND_CELLS_BATCH = 1 << 18;
+// pair_kernel, trio_kernel, general_kernel and rest_kernel) or all to octet_kernel,
+// which takes short lists by octets and long ones by threads.  Five kernels a step pay
+// where many cells are listed, which the host does not know: it follows the size.  us a
+// step, octet_kernel / by kind, after 20, 200 and 1000 steps: 80 x 80 x 80 33 / 40, 34 /
+// 41, 47 / 48; 300 x 60 x 28 45 / 47, 47 / 50, 62 / 61; 160 x 160 x 32 46 / 49, 49 / 52,
+// 68 / 66; 150 x 117 x 90 45 / 47, 47 / 50, 68 / 61; 128 x 128 x 128 46 / 49, 50 / 52, 69 /
+// 63.  Batches of 32 x 32 x 64, after 20 and 800 steps: 3 of them 23 / 36, 16 / 39, 12 of
+// them 39 / 44, 34 / 42.  Isotropic, one kernel either way, 10 steps with dense output: 45 x
+// 45 x 90 361 / 344, 64 x 64 x 64 425 / 356; a batch of 4 335 / 207.
+constexpr int64_t KIND_CELLS = 7 << 17, KIND_CELLS_ISOTROPIC = 1 << 19, KIND_PLANE_ISOTROPIC = 2000,
+                  KIND_CELLS_BATCH = 1 << 20;
 bool by_kind(const Params &P) {
-    return P.cells >= KIND_CELLS || (int64_t)P.nx * P.ny >= (P.use_aniso ? KIND_PLANE : KIND_PLANE_ISOTROPIC);
+    return P.use_aniso ? P.cells >= KIND_CELLS
+                       : P.cells >= KIND_CELLS_ISOTROPIC || (int64_t)P.nx * P.ny >= KIND_PLANE_ISOTROPIC;
 }
 bool by_kind_batch(const Params &P) { return P.cells >= KIND_CELLS_BATCH || !P.use_aniso; }
 
@@ -2287,8 +2512,8 @@ void launch_step(const In &in, const Out &out, const Mats &M, const Params &P, c
     else if (T.sweep_zb == 8) SWEEP_LAUNCH(8);
     else SWEEP_LAUNCH(4);
 #undef SWEEP_LAUNCH
-    if (!by_kind(P)) {  // 8 blocks of 128 threads are resident per SM
-        launch_early(P.sym_normals ? octet_kernel<S, AMAX, 4> : octet_kernel<S, AMAX, 8>, sms * 8, dim3(128), s, in,
+    if (!by_kind(P)) {
+        launch_early(P.sym_normals ? octet_kernel<S, AMAX, 4> : octet_kernel<S, AMAX, 8>, sms * OCTET_BLOCKS, dim3(128), s, in,
                      out, M, P, Q, parity, err);
         return;
     }
@@ -2300,8 +2525,8 @@ void launch_step(const In &in, const Out &out, const Mats &M, const Params &P, c
     launch_side_by_side(
         s,
         [&](cudaStream_t st) {
-            launch_early(P.sym_normals ? trio_kernel<S, 4> : trio_kernel<S, 8>, g_iface, dim3(T.iface_threads), st, in,
-                         out, M, P, Q, parity);
+            launch_early(P.sym_normals ? trio_kernel<S, AMAX, 4> : trio_kernel<S, AMAX, 8>, g_iface, dim3(T.iface_threads),
+                         st, in, out, M, P, Q, parity, err);
             launch_early(general_kernel<S>, g_general, dim3(T.general_threads), st, in, out, M, P, Q, parity);
         },
         [&](cudaStream_t st) {
@@ -2448,7 +2673,7 @@ void launch_batched(const In &in, const Out &out, const Mats &M, const Params &P
     const dim3 b_iface(T.iface_threads), b_general(T.general_threads);
     const bool sym = P0.sym_normals;
     if (!by_kind_batch(P0)) {
-        launch_early(sym ? batched_octet_kernel<S, AMAX, 4> : batched_octet_kernel<S, AMAX, 8>, sms * 8, dim3(128), s,
+        launch_early(sym ? batched_octet_kernel<S, AMAX, 4> : batched_octet_kernel<S, AMAX, 8>, sms * OCTET_BLOCKS, dim3(128), s,
                      in, out, M, P0, inst, n_inst, Q, parity, err);
         return;
     }
