@@ -1882,25 +1882,14 @@ __global__ void from_dense_kernel(const T *__restrict__ phi, int N, int nx, int 
     if (ovf) atomicOr(err, MPF3D_DEV_SLOT_OVERFLOW);
 }
 
-// compact -> dense [N][nx][ny][nz], four cells along z per thread, for nz a
-// multiple of 4 and aligned fields.  Bound by the N planes it writes, to HBM or
-// over the CPU-GPU link: each is written once, phase by phase beside the cells'
-// ascending lists, 16 bytes per thread and store, past the caches.  256^3 with 65
-// phases: 671 us (6.5 TB/s), with cached stores 727, by the kernel below 743;
-// 128^3 with 33 to pinned memory: 1432 us against 1499.  One or two cells per
-// thread in this form are slower than the kernel below (832; 150 x 117 x 90 with 33
-// phases 71 against 64).
-__device__ __forceinline__ void store_cells(float *p, const float (&v)[4]) {
-    __stcs((float4 *)p, make_float4(v[0], v[1], v[2], v[3]));
-}
-__device__ __forceinline__ void store_cells(double *p, const double (&v)[4]) {
-    __stcs((double2 *)p, make_double2(v[0], v[1]));
-    __stcs((double2 *)p + 1, make_double2(v[2], v[3]));
-}
-
-template <typename T, int S>
+// compact -> dense float32 [N][nx][ny][nz], four cells along z per thread, for nz a
+// multiple of 4, aligned fields and the cases of by_four_cells.  Bound by the N planes
+// it writes, to HBM or over the CPU-GPU link: each is written once, phase by phase beside
+// the cells' ascending lists, 16 bytes per store, past the caches.  256^3 with 65 phases:
+// 671 us (6.5 TB/s), with cached stores 727, by the kernel below 743.
+template <int S>
 __global__ void to_dense_kernel(In in, int N, int nx, int ny, int nz, uint32_t stride, uint32_t base,
-                                T *__restrict__ phi) {
+                                float *__restrict__ phi) {
     constexpr int V = 4;
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     const int m = blockIdx.y * blockDim.y + threadIdx.y;
@@ -1922,16 +1911,16 @@ __global__ void to_dense_kernel(In in, int N, int nx, int ny, int nz, uint32_t s
         val[j] = c > 1 ? __ldg(in.val + stride + q[j]) : 0.0f;
         left[j] = c - 2;
     }
-    T *dst = phi + ((int64_t)l * ny + m) * nz + k;
+    float *dst = phi + ((int64_t)l * ny + m) * nz + k;
     for (int g = 0; g < N; ++g, dst += plane) {
-        T v[V];
+        float v[V];
         bool hit = false;
 #pragma unroll
         for (int j = 0; j < V; ++j) {
-            v[j] = id[j] == g ? (T)cur[j] : (T)0;
+            v[j] = id[j] == g ? cur[j] : 0.0f;
             hit = hit || id[j] == g;
         }
-        store_cells(dst, v);
+        __stcs((float4 *)dst, make_float4(v[0], v[1], v[2], v[3]));
         if (!hit) continue;
 #pragma unroll
         for (int j = 0; j < V; ++j) {
@@ -1949,8 +1938,8 @@ __global__ void to_dense_kernel(In in, int N, int nx, int ny, int nz, uint32_t s
     }
 }
 
-// One cell per thread, for the other nz and unaligned fields: the planes zeroed,
-// then the few stored phases written over them.
+// One cell per thread, for the others: the planes zeroed, then the few stored phases
+// written over them.
 template <typename T, int S>
 __global__ void to_dense_each_kernel(In in, int N, int nx, int ny, int nz, uint32_t stride, uint32_t base,
                                      T *__restrict__ phi) {
@@ -2328,12 +2317,27 @@ dim3 zfast_grid(int nx, int ny, int nz, dim3 b) {
 }
 
 
+// Whether to_dense_kernel writes a float32 field, four cells a thread.  Over the CPU-GPU
+// link its wide stores win at every size (us, a cell / four cells a thread: 32^3 with 9
+// phases 15 / 13, 512 x 512 x 8 with 9 736 / 435, 128^3 with 33 1500 / 1436).  In device memory
+// it wants many planes and whole rows of threads along z (32^3 with 9 phases 6.8 / 8.8, 512 x
+// 512 x 8 with 9 58 / 64, 128 x 128 x 64 with 33 31 / 36, 64^3 with 301 62 / 58, 128^3 with 33
+// 52 / 49).  Float64 is not for it: a warp's stores of four cells leave gaps (128^3 with 33 in
+// device memory 93 / 163, over the link 2975 / 7211).
+bool by_four_cells(int64_t values, int nz, const void *phi) {
+    cudaPointerAttributes at{};
+    const bool known = cudaPointerGetAttributes(&at, phi) == cudaSuccess;
+    if (!known) cudaGetLastError();
+    if (known && at.type == cudaMemoryTypeHost) return true;
+    return values >= (int64_t)1 << 26 && nz >= 64;
+}
+
 template <typename T, int S>
 void launch_to_dense(const In &in, int N, int nx, int ny, int nz, uint32_t stride, uint32_t base, T *phi,
                      cudaStream_t s) {
     const dim3 b(16, 4, 4), each(32, 4, 2);
-    if (nz % 4 == 0 && (uintptr_t)phi % 16 == 0)
-        to_dense_kernel<T, S><<<zfast_grid(nx, ny, nz / 4, b), b, 0, s>>>(in, N, nx, ny, nz, stride, base, phi);
+    if (sizeof(T) == 4 && nz % 4 == 0 && (uintptr_t)phi % 16 == 0 && by_four_cells((int64_t)nx * ny * nz * N, nz, phi))
+        to_dense_kernel<S><<<zfast_grid(nx, ny, nz / 4, b), b, 0, s>>>(in, N, nx, ny, nz, stride, base, (float *)phi);
     else
         to_dense_each_kernel<T, S><<<zfast_grid(nx, ny, nz, each), each, 0, s>>>(in, N, nx, ny, nz, stride, base, phi);
 }
