@@ -19,6 +19,8 @@ import os
 
 from . import _lib
 
+# of the step's kernels: a pick cached for others is not applied to these
+KERNELS = 3
 DEFAULT = (4, 8, 16, 128, 16, 128)
 SWEEP = [(zb, by) for zb in (2, 4, 8) for by in (4, 8, 16)]
 QUEUE = [(g, gt, i, it) for (g, gt), (i, it) in itertools.product([(4, 256), (8, 256), (16, 128), (32, 128)],
@@ -42,7 +44,7 @@ def key_of(solver) -> str:
 
     name = torch.cuda.get_device_name(solver.device)
     return (f"{name}|{solver.nx}x{solver.ny}x{solver.nz}|N{solver.N}|S{solver.slots}|"
-            f"a{int(solver.anisotropy)}t{int(solver.torque)}")
+            f"a{int(solver.anisotropy)}t{int(solver.torque)}|k{KERNELS}")
 
 
 def _load() -> dict:
@@ -145,7 +147,7 @@ def tune_batched(batch, steps: int = 8, use_cache: bool = True) -> dict:
 
     name = torch.cuda.get_device_name(batch.device)
     key = (f"batched|{name}|n{batch.n}|cells{batch.total_cells}|S{batch.slots}|"
-           f"a{int(batch.anisotropy)}t{int(batch.torque)}")
+           f"a{int(batch.anisotropy)}t{int(batch.torque)}|k{KERNELS}")
     db = _load() if use_cache else {}
     if use_cache and key in db:
         batch.tuning = make(db[key]["config"])
