@@ -294,10 +294,13 @@ def run_reference(args, rank):
     print(json.dumps(line), flush=True)
 
 
-def launches_per_step(cells):
-    """Kernels of a compact step with anisotropy: sweep and octet_kernel; sweep,
-    pair, trio, general and rest kernels on large domains (every workload here)."""
-    return 5 if cells >= 1 << 19 else 2
+def launches_per_step(grid=None, batch_cells=0):
+    """Kernels of a compact step with anisotropy, of a domain or of a batch: sweep, pair,
+    trio, general and rest kernels, or on small ones sweep and octet_kernel."""
+    from mpf3d import _lib
+    L = _lib.lib()
+    return 5 if (L.mpf3d_compact_step_by_kind(*grid, 1) if grid else
+                 L.mpf3d_batched_step_by_kind(batch_cells, 1)) else 2
 
 
 def config_dict(args):
@@ -827,7 +830,7 @@ def bicrystal_run(args, dev, rank=0, world=1):
             "gb_inclination_deg": {"finite": int(np.isfinite(ang).sum()),
                                    "median_abs": float(np.nanmedian(np.abs(ang))) if np.isfinite(ang).any()
                                    else None},
-            "launches_per_step": launches_per_step(b.total_cells), "graph_steps": 50,
+            "launches_per_step": launches_per_step(batch_cells=b.total_cells), "graph_steps": 50,
             "launch_shape": {"work_list_kernels": list(tuned["config"][2:]), "ms_per_step_tuned": tuned["ms_per_step"],
                              "ms_per_step_default": tuned["default_ms_per_step"]} if tuned else None}
 
@@ -842,7 +845,7 @@ def emit(args, rank, world, value, ms, cells, t_e2e, in_bytes, out_bytes, achiev
                 "e2e": {"value": cells * args.steps * world / t_e2e, "unit": UNIT,
                         "h2d_bytes_per_step": in_bytes / args.steps,
                         "d2h_bytes_per_step": out_bytes / args.steps},
-                "gpu_launches": launches_per_step(cells) * args.steps,
+                "gpu_launches": launches_per_step(GRID) * args.steps,
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                              "frac": achieved / peak, "traffic": traffic,
                              "peak_source": peak_kind,
@@ -904,7 +907,7 @@ def run_c3(args):
                                    "anisotropy+torque, uniform cooling, FP32 compact, started from the owner map",
                        "slots": s.slots, "state_bytes_per_buffer": s.state_bytes()},
             "setup_s": setup, "stored_phases_per_cell_end": float(s.stored_counts().double().mean().item()),
-            "clocks": clk.summary(), "gpu_launches": launches_per_step(cells) * args.steps,
+            "clocks": clk.summary(), "gpu_launches": launches_per_step((nx, ny, nz)) * args.steps,
             "launch_shape": {"config": list(tuned["config"]), "sweep_tma": bool(s.sweep_tma),
                              "ms_per_step_tuned": tuned["ms_per_step"],
                              "ms_per_step_default": tuned["default_ms_per_step"]} if tuned else None}

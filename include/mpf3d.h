@@ -228,6 +228,12 @@ int mpf3d_compact_step_tuned(const uint32_t *head, const uint16_t *idx, const fl
                              uint32_t *work_items, uint32_t *work_count, int parity, int32_t *err,
                              void *stream, const mpf3d_tuning *tuning, uint8_t *tile_flags, int options);
 
+/* Whether a step of this domain, or of a batch of this many cells, runs its work lists
+ * by kernels per kind of cell, whose grids mpf3d_tuning shapes (1), or by one kernel
+ * with a grid of its own (0): the general_ and iface_ fields then change nothing. */
+int mpf3d_compact_step_by_kind(int nx, int ny, int nz, int enable_anisotropy);
+int mpf3d_batched_step_by_kind(uint32_t total_cells, int enable_anisotropy);
+
 /* options of mpf3d_compact_step_tuned */
 #define MPF3D_STEP_MULTI_LIST 1 /* interface cells whose neighbourhood holds two or more solids
                                  * get a work list of their own at

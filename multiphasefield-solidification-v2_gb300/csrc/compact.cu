@@ -2790,6 +2790,24 @@ extern "C" int mpf3d_compact_step(const uint32_t *cnt, const uint16_t *idx, cons
                                     nullptr, 0);
 }
 
+extern "C" int mpf3d_compact_step_by_kind(int nx, int ny, int nz, int enable_anisotropy) {
+    if (!dims_ok(nx, ny, nz)) return 0;
+    Params P;
+    memset(&P, 0, sizeof P);
+    P.nx = nx; P.ny = ny; P.nz = nz;
+    P.cells = (int64_t)nx * ny * nz;
+    P.use_aniso = enable_anisotropy != 0;
+    return by_kind(P) ? 1 : 0;
+}
+
+extern "C" int mpf3d_batched_step_by_kind(uint32_t total_cells, int enable_anisotropy) {
+    Params P;
+    memset(&P, 0, sizeof P);
+    P.cells = total_cells;
+    P.use_aniso = enable_anisotropy != 0;
+    return by_kind_batch(P) ? 1 : 0;
+}
+
 extern "C" int64_t mpf3d_compact_tile_flags_len(int nx, int ny, int nz) {
     if (!dims_ok(nx, ny, nz)) return 0;
     return 2 * (int64_t)tiles_of<2>(nx, ny, nz);

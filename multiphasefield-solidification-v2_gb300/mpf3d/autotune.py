@@ -2,8 +2,8 @@
 
 The reference launches every kernel with a fixed [4, 4, 4] block
 (config_3d.yaml gpu.threads_per_block).  Here the shape -- cells per sweep
-thread along z, sweep block height, the grid and block sizes of the two
-work-list kernels, and whether the sweep stages its heads in shared memory by
+thread along z, sweep block height, the grid and block sizes of the
+work-list kernels (where a step has several), and whether the sweep stages its heads in shared memory by
 TMA -- is searched per problem (grid, phases, slots, model
 switches, GPU) by timing each candidate on the solver's own state with CUDA
 events, restoring the state before every trial.  All shapes compute identical
@@ -114,8 +114,10 @@ def tune(solver, steps: int = 8, use_cache: bool = True) -> dict:
             trials[str(cfg)] = time_config(solver, cfg, steps)
         if trials[str(cfg)] < best_ms:
             best, best_ms = cfg, trials[str(cfg)]
-    # stage 2: the work-list kernels with the best sweep shape
-    for q in QUEUE:
+    # stage 2: the work-list kernels with the best sweep shape (one kernel with a grid of
+    # its own on small domains)
+    by_kind = _lib.lib().mpf3d_compact_step_by_kind(solver.nx, solver.ny, solver.nz, int(solver.anisotropy))
+    for q in QUEUE if by_kind else ():
         cfg = best[:2] + q
         if str(cfg) not in trials:
             trials[str(cfg)] = time_config(solver, cfg, steps)
@@ -139,7 +141,7 @@ def tune(solver, steps: int = 8, use_cache: bool = True) -> dict:
 
 
 def tune_batched(batch, steps: int = 8, use_cache: bool = True) -> dict:
-    """Search the grid and block sizes of the batched step's two work-list
+    """Search the grid and block sizes of the batched step's work-list
     kernels (the QUEUE candidates) on the batch's own state, restored after
     every trial; sets batch.tuning.  Cached per (GPU, instance count, total
     cells, slots, model switches)."""
@@ -181,7 +183,8 @@ def tune_batched(batch, steps: int = 8, use_cache: bool = True) -> dict:
     base = trial(DEFAULT)
     trials[str(DEFAULT)] = base
     best, best_ms = DEFAULT, base
-    for q in QUEUE:
+    by_kind = _lib.lib().mpf3d_batched_step_by_kind(batch.total_cells, int(batch.anisotropy))
+    for q in QUEUE if by_kind else ():
         cfg = DEFAULT[:2] + q
         if str(cfg) not in trials:
             trials[str(cfg)] = trial(cfg)
