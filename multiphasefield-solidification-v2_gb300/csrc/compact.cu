@@ -1684,10 +1684,12 @@ __device__ __forceinline__ void for_octets(const Queue &Q, uint32_t cells, int p
 // each, one after the other.  For the same reason a block takes runs of RUN
 // items from distant parts of the range; PER: items that make another block
 // worth starting.
-// With EACH, a block that is left with more than MANY_LEFT of them, and more than half of
-// its items, does them by each(item), one per thread (64 x 64 x 64 isotropic, 140 k cells
-// with 9 phases: 379 us a step by octets, 136 so).
-constexpr uint32_t LEFT_CELLS = 1024, MANY_LEFT = 96;
+// With EACH, a block that is left with more than MANY_LEFT of them, and more than a third
+// of its items, does them by each(item), one per thread.  isotropic_kernel, us a step, by
+// octets / threads with a block for every 256 items, 96 and half of them / as it is: 64^3 with
+// 146 k cells of 9 phases 380 / 130 / 108, 80^3 with 40 grains and 143 k cells listed 219 / 199 /
+// 128, with a front, 8 grains and 35 k 21 / 21 / 17; a block for every 64 items 298, 148, 17.
+constexpr uint32_t LEFT_CELLS = 1024, MANY_LEFT = 48;
 
 template <uint32_t RUN, uint32_t PER, bool EACH, class Get, class Take, class Rest, class Each>
 __device__ __forceinline__ void for_items(uint32_t n, Get &&get, Take &&take, Rest &&rest, Each &&each) {
@@ -1708,7 +1710,7 @@ __device__ __forceinline__ void for_items(uint32_t n, Get &&get, Take &&take, Re
         }
         __syncthreads();
         const uint32_t m = n_left;
-        if (EACH && m > MANY_LEFT && 2u * m > (min(at0, n) - first) / blocks) {
+        if (EACH && m > MANY_LEFT && 3u * m > (min(at0, n) - first) / blocks) {
             for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) each(left[i]);
         } else {
             for (uint32_t w = warp; w * 4u < m; w += blockDim.x >> 5)
@@ -1830,7 +1832,7 @@ __global__ void __launch_bounds__(256, 3)
     isotropic_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity, int32_t *__restrict__ err) {
     wait_for_previous();
     const OctetLane O;
-    for_items<32, 256, true>(
+    for_items<32, 128, true>(
         *(volatile uint32_t *)(Q.count + 2 * parity), [&](uint32_t i) { return Q.items[i]; },
         [&](uint32_t c) {
             const Place at(c, P.nx, P.ny);
@@ -2156,7 +2158,7 @@ __global__ void __launch_bounds__(256, 3)
     batched_isotropic_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity, int32_t *__restrict__ err) {
     wait_for_previous();
     const OctetLane O;
-    for_items<32, 256, true>(
+    for_items<32, 128, true>(
         *(volatile uint32_t *)(Q.count + 2 * parity), [&](uint32_t i) { return Q.items[i]; },
         [&](uint32_t c) {
             const mpf3d_instance I = inst[find_instance_by_cell(inst, n_inst, c)];
