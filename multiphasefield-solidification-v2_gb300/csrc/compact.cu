@@ -73,10 +73,6 @@ struct Params {
 };
 
 
-__device__ __forceinline__ int64_t cell_of(const Params &P, int l, int m, int k) {
-    return ((int64_t)k * P.ny + m) * P.nx + l;
-}
-
 // max |cos| between a gradient and the grain's 8 rotated {111} normals, with
 // the signed cosine and the winning normal (best_cos_from_grad_3d :110-134,
 // facet_cos_and_nxyz_from_grad :251-301)
@@ -1498,7 +1494,7 @@ __device__ __forceinline__ bool mbar_wait_ns(uint32_t bar, uint32_t parity, uint
 // domain are never read (the clamped neighbour is the cell itself).  A copy
 // that does not land within 1 s sets MPF3D_DEV_STAGING_TIMEOUT and the block
 // waits once more before it leaves.  Same results as sweep_kernel.
-template <int S, int AMAX, int ZB>
+template <int ZB>
 __global__ void __launch_bounds__(512, 3) sweep_kernel_tma(const __grid_constant__ CUtensorMap map, In in, Out out,
                                                          Params P, Queue Q, int parity, Tiles T,
                                                          int32_t *__restrict__ err) {
@@ -2507,7 +2503,7 @@ void launch_step(const In &in, const Out &out, const Mats &M, const Params &P, c
     do {                                                                                                           \
         const dim3 grid((P.nx + 31) / 32, (P.ny + by - 1) / by, (P.nz + ZB - 1) / ZB);                             \
         const Tiles tl{tile_flags, (P.nx + 31) / 32, (P.nz + ZB - 1) / ZB, tiles_of<ZB>(P.nx, P.ny, P.nz)};       \
-        if (tma) sweep_kernel_tma<S, AMAX, ZB><<<grid, blk, 0, s>>>(map, in, out, P, Q, parity, tl, err);          \
+        if (tma) sweep_kernel_tma<ZB><<<grid, blk, 0, s>>>(map, in, out, P, Q, parity, tl, err);          \
         else {                                                                                                     \
             const uint32_t chunks = grid.x * grid.y * grid.z;                                                      \
             launch_early(sweep_kernel<ZB>, sweep_blocks(chunks, by, sms), blk, s, in, out, P, Q, parity, tl,       \
