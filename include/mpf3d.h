@@ -167,10 +167,11 @@ int mpf3d_compact_active_count(const uint32_t *head, const uint16_t *idx, int sl
  * the work-list kernels of the step) and work_count uint32[4],
  * zeroed once before the first step; `parity` alternates 0/1 on consecutive
  * steps so no reset is needed in between.  Cells must number fewer than 2^31.
- * Streams: with anisotropy on and a domain that is not small, the kernel of the
- * one-solid interface cells runs on a library-owned second stream, beside the
- * kernels of the other lists, forked from and joined back to `stream` by events; to the caller the step is ordered on `stream` like one
- * kernel.  Each caller stream of each device gets its own second stream and
+ * Streams: with anisotropy on and kernels by kind of cell
+ * (mpf3d_compact_step_by_kind), the kernel of the one-solid interface cells runs on
+ * a library-owned second stream, beside the kernels of the other lists, forked from
+ * and joined back to `stream` by events; to the caller the step is ordered on
+ * `stream` like one kernel.  Each caller stream of each device gets its own second stream and
  * event pair, created by its first such call made outside a stream capture;
  * a call inside a capture before that launches them all on `stream`.
  * Steps that callers issue on independent streams therefore stay

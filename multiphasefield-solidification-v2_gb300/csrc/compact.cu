@@ -7,9 +7,10 @@
 // cell's active-phase list from the stored lists of the cell and its 6 face
 // neighbours, evaluate the anisotropic interface, torque and kinetic terms and
 // the pair sums, clip, renormalise and write only the phases that stay positive.
-// Small domains have one list kernel (octet_kernel), large ones one per kind of
-// cell: pair_kernel, trio_kernel, general_kernel and, for what those leave,
-// rest_kernel (isotropic_kernel alone without anisotropy).
+// Small domains have one list kernel (octet_kernel: eight lanes per cell, or one thread
+// where the lists are long), large ones one per kind of cell: pair_kernel, trio_kernel,
+// general_kernel and, for what those leave, rest_kernel (isotropic_kernel alone without
+// anisotropy).
 //
 // State layout in HBM (x fastest, so a warp of 32 threads along x reads
 // 32 consecutive entries of each array and an interface -- normal to z --
@@ -400,17 +401,18 @@ __device__ __forceinline__ void interface_terms(const Params &P, const Stencil &
     center_terms(P, g0, t0, L, st.hxy, st.hxz, st.hyz, flux, div, lap_sl, b_sl);
 }
 
-// Three forms of the update of a queued cell give the same bits:
+// Four forms of the update of a queued cell give the same bits:
 //   pair_cell   one thread, a neighbourhood of the liquid and one solid
 //   trio_cell   one thread, a neighbourhood of up to three phases
 //   octet_cell  eight lanes, any neighbourhood
+//   any_cell    one thread, any neighbourhood, its phases in local memory
 // The first two take most cells of a large domain: no per-phase arrays in local
 // memory, and the records in one or two rounds of loads.  What they leave, and
 // everything on small domains, where a step is one cell's latency, goes to the
-// third.  A 256^3 step with 64 grains (0.57 M general cells, 0.30 M pairs, 73 k
-// others, 13 k of them beyond three phases): pairs 29 us, general 28, trios 16,
-// rest 24; with one thread per cell for any neighbourhood, its arrays in local
-// memory, the two list kernels took 150 us.  By octets alone the lists take 292.
+// third, or to the fourth where that is many cells.  A 256^3 step with 64 grains (0.57
+// M general cells, 0.30 M pairs, 73 k others, 13 k of them beyond three phases), each
+// kernel by itself with cold caches: pairs 24 us, general 24, trios 23, rest 25; by
+// any_cell alone the two list kernels took 150 us, by octets alone the lists take 292.
 
 // Update of an interface cell whose neighbourhood holds the liquid and one
 // solid, as the sweep's list 1 does where it split the lists: no merge, and only
@@ -951,8 +953,8 @@ __device__ __forceinline__ bool octet_phases(const In &in, const Out &out, const
     return true;
 }
 
-// the cells of a warp by up to 8 phases, one per lane; where one has more, by
-// AMAX (out of line: its arrays would cost the common case registers)
+// the cells of a warp by up to 8 phases, one per lane; where one has more, by AMAX (whose
+// arrays cost rest_kernel with 16 slots about 300 bytes of spills)
 template <int S, int AMAX, int NT>
 __device__ __forceinline__ void octet_many(const In &in, const Out &out, const Mats &M, const Params &P,
                                         int32_t *__restrict__ err, const OctetLane &O, bool active, int l, int m,
@@ -1734,8 +1736,8 @@ struct Place {
     }
 };
 
-// Kernel 2 of a step on small domains: eight lanes per cell.  NT: normals per
-// grain (4 or 8, from P.sym_normals).
+// Kernel 2 of a step on small domains: eight lanes per cell, or one thread where the
+// lists are long.  NT: normals per grain (4 or 8, from P.sym_normals).
 template <int S, int AMAX, int NT>
 __global__ void __launch_bounds__(128, OCTET_BLOCKS) octet_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity,
                                                        int32_t *__restrict__ err) {
@@ -1752,7 +1754,7 @@ __global__ void __launch_bounds__(128, OCTET_BLOCKS) octet_kernel(In in, Out out
 }
 
 // The work-list kernels on large domains: list 1 by pair_cell, where the sweep
-// kept it to pairs, beside lists 2 and 0 by trio_cell.
+// kept it to pairs, on a second stream beside lists 2 and 0 by trio_cell.
 template <int NT>
 __global__ void __launch_bounds__(128, 5) pair_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity) {
     const uint32_t n = *(volatile uint32_t *)(Q.count + 2 * parity + 1);
@@ -1790,7 +1792,7 @@ __global__ void __launch_bounds__(128, 4) trio_kernel(In in, Out out, Mats M, Pa
     }
 }
 
-// list 0: grain boundaries and junctions, beside the above
+// list 0: grain boundaries and junctions, after trio_kernel on its stream
 template <int S>
 __global__ void __launch_bounds__(256, 4) general_kernel(In in, Out out, Mats M, Params P, Queue Q, int parity) {
     wait_for_previous();
@@ -2114,7 +2116,7 @@ __global__ void __launch_bounds__(128, 4) batched_trio_kernel(In in, Out out, Ma
     }
 }
 
-// list 0: grain boundaries and junctions, beside the above
+// list 0: grain boundaries and junctions
 template <int S>
 __global__ void __launch_bounds__(256, 4) batched_general_kernel(In in, Out out, Mats M, Params P0, const mpf3d_instance *__restrict__ inst, int n_inst, Queue Q, int parity) {
     wait_for_previous();
@@ -2356,8 +2358,8 @@ int to_dense(const In &in, int slots, int N, int nx, int ny, int nz, uint32_t st
     return cudaGetLastError() == cudaSuccess ? MPF3D_OK : MPF3D_ERR_CUDA;
 }
 
-// A second stream of one device, on which pair_kernel runs beside trio_kernel
-// and general_kernel.  They read only what the sweep wrote and write disjoint
+// A second stream of one device, on which pair_kernel runs beside trio_kernel and then
+// general_kernel on the caller's.  They read only what the sweep wrote and write disjoint
 // cells, and fill each other's idle issue slots.  Created on first use outside a
 // stream capture; the fork/join is enqueued under the mutex so that callers
 // on other host threads cannot interleave their event records with it.
@@ -2668,9 +2670,9 @@ void launch_batched(const In &in, const Out &out, const Mats &M, const Params &P
     const int sms = sms_of_current_device();
     launch_early(batched_sweep_kernel, sweep_blocks((uint32_t)n_tiles, 8, sms), dim3(32, 8), s, in, out, P0, inst,
                  n_inst, Q, parity, tile_flags, (uint32_t)n_tiles);
-    // one stream: the side-by-side launch of the compact step measured no
-    // gain here; the work-list grids come from T (the sweep's 32 x 8 x 4
-    // tiles are fixed by the instance table)
+    // one stream: the side-by-side launch of the compact step measured no gain here when
+    // there were two list kernels (not measured with these); the work-list grids come from
+    // T (the sweep's 32 x 8 x 4 tiles are fixed by the instance table)
     const int g_iface = sms * T.iface_blocks_per_sm, g_general = sms * T.general_blocks_per_sm;
     const dim3 b_iface(T.iface_threads), b_general(T.general_threads);
     const bool sym = P0.sym_normals;

@@ -26,8 +26,8 @@
 // us for 65,536 rows; the weights' way from L2, 128 KB per tile and layer with
 // 64 KB in flight per SM, adds the rest.  Measured on GB300: forward of 65,536
 // rows 125 -> 41 us (one CTA per SM with a ring of 8 chunks: 66 us); an
-// optimiser step on 512 rows 843 -> 56 us on the device (forward 20, chain 22,
-// weight gradients 7.5).  For few rows the time is that of one tile, about 5
+// optimiser step on 512 rows, call to call, 843 -> 83 to 91 us (each kernel by itself
+// with cold caches: forward 24 us, gradient chain 36, weight gradients 9).  For few rows the time is that of one tile, about 5
 // us a layer, and the ring of 8 hides the weights.
 // Every wait is bounded; a wait that runs out ends the CTA's work as in mlp.cu:
 // the issued MMAs and copies are waited for (bounded), the outputs of the
@@ -95,9 +95,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 }
 
 // silu_grad without the division's branch per value: 1 / d for d >= 1 by one
-// Newton step from the approximate reciprocal (Markstein's correction, FMA
-// residual), which gives the rounded quotient there; near overflow of d the
-// approximation itself
+// Newton step from the approximate reciprocal (FMA residual), within one unit in the
+// last place; near overflow of d the approximation itself
 __device__ __forceinline__ float silu_slope(float z) {
     const float d = 1.0f + __expf(-z);
     const float r = __fdividef(1.0f, d);

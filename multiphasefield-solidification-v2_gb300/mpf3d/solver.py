@@ -1,10 +1,10 @@
-"""Compact FP32 solver: the fused one-kernel-per-step tier.
+"""Compact FP32 solver: a sweep and the kernels of its work lists per step.
 
 ``CompactSolver`` owns a double-buffered compact state on one GPU (see
 include/mpf3d.h for the layout) and advances it with ``mpf3d_compact_step``.
 It replaces the reference's driver loop (run_randommode_3d.py:267-287:
-temperature kernel, APT kernel, update kernel, buffer swap) with one launch
-per step; dense phi is only materialised on request (``to_dense``).
+temperature kernel, APT kernel, update kernel, buffer swap); dense phi is only
+materialised on request (``to_dense``).
 
 Device memory comes from torch (plumbing only); all compute is in
 libmpf3d.so.
