@@ -10,11 +10,11 @@ torch = pytest.importorskip("torch")
 BOX, GRAINS, STEPS = (22, 20, 40), 8, 40
 
 
-def solver(copies, antipodal=True, **kw):
+def solver(copies, antipodal=True, box=BOX, **kw):
     """A melt undercooled so far that every grain's phase grows everywhere."""
     from mpf3d import inputs
     from mpf3d.solver import CompactSolver
-    case = inputs.voronoi_case(*BOX, GRAINS, 8, seed=9, orientation_seed=3, undercooling=2.0)
+    case = inputs.voronoi_case(*box, GRAINS, 8, seed=9, orientation_seed=3, undercooling=2.0)
     n111 = case.n111
     if not antipodal:
         n111 = np.random.default_rng(1).standard_normal(n111.shape).astype(np.float32)
@@ -45,6 +45,17 @@ def test_copies_step_as_the_box(copies, slots, antipodal, anisotropy):
         assert sum(lists(box)) < 40000 and lists(box)[2] < 16384  # octets
         _, one, several = lists(many)
         assert several > (60000 if copies == (8, 7) else 16384) and several > 8 * one
+
+
+def test_long_isotropic_lists_of_a_narrow_domain():
+    """Too small a plane for isotropic_kernel: octet_kernel's threads on list 0 alone."""
+    kw = dict(box=(22, 20, 90), slots=16, anisotropy=False)
+    box, many = solver((1, 1), **kw), solver((2, 2), **kw)
+    for steps in (1, 79):
+        box.step(steps)
+        many.step(steps)
+        assert torch.equal(many.to_dense(host=False), box.to_dense(host=False).repeat(1, 2, 2, 1))
+    assert lists(box)[0] < 49152 < lists(many)[0]
 
 
 @pytest.mark.parametrize("copies", [(3, 3), (8, 7)])
